@@ -272,9 +272,9 @@ def work(case):
     n = _APPLICATIONS[call]
     w = _operator_work(case, case["inner"] or case["prec"], 2)
     # the operator's bytes each application, and the solver's vectors: a CG half-iteration passes over about 4
-    # spinors, a BiCGStab half-iteration over about 9, a multishift one over every shift's x and p, read and written
-    vectors = {"cg": 4, "richardson": 9}.get(call, 2 * case["shifts"]) * case["nrhs"]
-    return {"bytes": n * (w["bytes"] + vh * vectors * _spinor_bytes(case["inner"] or case["prec"])),
+    # spinors, a BiCGStab half-iteration over about 9; a multishift solve also writes each solution once
+    spinor = vh * case["nrhs"] * _spinor_bytes(case["inner"] or case["prec"])
+    return {"bytes": n * (w["bytes"] + {"richardson": 9}.get(call, 4) * spinor) + case["shifts"] * spinor,
             "flops": n * w["flops"]}
 
 
