@@ -225,9 +225,17 @@ void launch_clover_out(int prec, Geom g, HostLayout L, void *host, const void *d
   QPX_PREC_SWITCH(prec, (clover_out_kernel<P><<<grid, QPX_BLOCK, 0, st>>>(g, L, host, dev, stride, vpc, nr)));
 }
 
-void launch_mshift(int prec, const MShiftArgs &a, dim3 grid, cudaStream_t st)
+void launch_mshift_base(int prec, int vh, int nshift, int slot, SpinorArg r, SpinorArg p0, const SolverState *state,
+                        MShiftHist *hist, dim3 grid, cudaStream_t st)
 {
-  QPX_PREC_SWITCH(prec, (mshift_update_kernel<P><<<grid, QPX_BLOCK, 0, st>>>(a)));
+  QPX_PREC_SWITCH(prec, (mshift_base_kernel<P><<<grid, QPX_BLOCK, 0, st>>>(vh, nshift, slot, r, p0, state, hist)));
+}
+
+void launch_mshift_update(int prec, const MShiftArgs &a, dim3 grid, cudaStream_t st)
+{
+  // whole sites (16-bit storage) or a site's chunks in blockIdx.y
+  QPX_PREC_SWITCH(prec, (mshift_update_kernel<P><<<dim3(grid.x, P::has_norm ? 1 : SpinorIO<P>::nchunk), QPX_BLOCK, 0,
+                                                   st>>>(a)));
 }
 
 bool launch_dslash_f64(int recon, int epi, int achi, const DslashShape &sh, const DslashArgs *a, dim3 grid,

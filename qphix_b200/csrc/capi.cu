@@ -12,6 +12,7 @@
 #include <cstring>
 #include <iterator>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -185,6 +186,7 @@ static void lattice_release(qphix_gpu_lattice_s *L)
   cudaFree(L->state);
   cudaFreeHost(L->h_state);
   if (L->grid_bar) cudaFree(L->grid_bar);
+  if (L->mshift_hist) cudaFree(L->mshift_hist);
   if (L->stream && L->owns_stream) cudaStreamDestroy(L->stream);
   delete L;
 }
@@ -1901,13 +1903,14 @@ SolverState &state_reset(qphix_gpu_lattice_s *lat, int nrhs, int max_iter)
 
 // Replays `step` (one solver iteration, kernels only) until the device raises
 // state->done.  The step is captured once into a CUDA graph.
+// `per_step`: solver iterations of one step (the host polls every 8).
 // `key` names everything the captured launches depend on (solver, operator
 // and field serial numbers, isign, cb); a graph captured under the same key
 // is replayed instead of captured again.
 template <typename Step>
-void run_iterations(qphix_gpu_lattice_s *lat, Step &&step, int max_iter, const std::string &key)
+void run_iterations(qphix_gpu_lattice_s *lat, Step &&step, int max_iter, const std::string &key, int per_step = 1)
 {
-  const int check = 8;
+  const int check = std::max(1, 8 / per_step);  // steps between polls
   bool use_graph = !env_flag("QPHIX_GPU_NO_GRAPH");
   cudaGraphExec_t exec = nullptr;
   unsigned long long nodes = 0;
@@ -1960,13 +1963,13 @@ void run_iterations(qphix_gpu_lattice_s *lat, Step &&step, int max_iter, const s
           g_launches += nodes;
         } else
           step();
-        launched++;
+        launched += per_step;
       }
       QPX_CUDA(cudaMemcpyAsync(&lat->h_state->done, &lat->state->done, sizeof(int), cudaMemcpyDeviceToHost,
                                lat->stream));
       QPX_CUDA(cudaStreamSynchronize(lat->stream));
       if (lat->h_state->done) break;
-      if (launched > max_iter + 2 * check) break;  // the device enforces max_iter; belt and braces
+      if (launched > max_iter + 2 * check * per_step) break;  // the device enforces max_iter; belt and braces
     }
   } catch (...) {
     if (exec && !cached) cudaGraphExecDestroy(exec);
@@ -2968,8 +2971,10 @@ extern "C" int qphix_gpu_solve_richardson(qphix_gpu_eo_op op_outer, qphix_gpu_eo
 // ---------------------------------------------------------------------------
 // multishift CG (include/qphix/minvcg.h:77-387): one M^dag M per iteration
 // for the base system; the per-shift zeta / beta recurrences run on the device
-// (FIN_MCG_*), r += b M^dag M p0 is fused into the second Dslash, and every
-// shifted x / p update plus p0 = r + a p0 is one multi-vector kernel.
+// (FIN_MCG_*), r + b M^dag M p0 is fused into the second Dslash and goes to
+// the next of `batch` residual buffers, p0 = r + a p0 is a kernel of its own,
+// and every shifted x / p update of `batch` iterations is one multi-vector
+// kernel (qpx_blas.cuh).
 static void solve_mshift(qphix_gpu_eo_op_s *op, qphix_gpu_field_s **x, qphix_gpu_field_s *rhs, int ns,
                          const double *shifts, const double *rsd, int max_iters, int isign, int cb, int *n_iters,
                          double *rsd_sq_final, unsigned long *mv_apps)
@@ -2986,16 +2991,27 @@ static void solve_mshift(qphix_gpu_eo_op_s *op, qphix_gpu_field_s **x, qphix_gpu
   require_same(rhs, op->gauge);
   auto *lat = rhs->lat;
   const int prec = rhs->prec;
-  Tmp r(lat, prec, 1), p0(lat, prec, 1), mp(lat, prec, 1), mmp(lat, prec, 1);
-  std::vector<Tmp *> ps;
-  for (int s = 0; s < ns; s++) ps.push_back(new Tmp(lat, prec, 1));
-  struct Free {
-    std::vector<Tmp *> &v;
-    ~Free()
-    {
-      for (auto *t : v) delete t;
-    }
-  } free_ps{ps};
+  Tmp p0(lat, prec, 1), mp(lat, prec, 1), mmp(lat, prec, 1);
+  std::vector<std::unique_ptr<Tmp>> ps, rs;
+  for (int s = 0; s < ns; s++) ps.emplace_back(new Tmp(lat, prec, 1));
+  rs.emplace_back(new Tmp(lat, prec, 1));
+  // A residual buffer per iteration of a batch: the update pass moves
+  // (4 ns + batch) / batch spinors per iteration (24^3x48 FP64, 16 shifts:
+  // 586 us in batches of 1).  For few shifts the buffers would outnumber the
+  // vectors they save passes over.  A device that is full gets the batch
+  // that fits.
+  const int want = ns >= 4 ? QPX_MSHIFT_BATCH : QPX_MSHIFT_BATCH / 2;
+  try {
+    while ((int)rs.size() < want) rs.emplace_back(new Tmp(lat, prec, 1));
+  } catch (const Error &e) {
+    if (e.code != QPHIX_GPU_ENOMEM) throw;
+    cudaGetLastError();  // the failed allocation, not a launch's error
+  }
+  int batch = 1;
+  while (2 * batch <= (int)rs.size()) batch *= 2;
+  if (!lat->mshift_hist) QPX_CUDA(cudaMalloc(&lat->mshift_hist, sizeof(MShiftHist)));
+  MShiftHist *hist = static_cast<MShiftHist *>(lat->mshift_hist);
+  qphix_gpu_field_s *r = *rs[0];
   double cp = norm2_host(rhs)[0];
   // r = p0 = p_s = rhs
   BlasCall cpy;
@@ -3060,41 +3076,52 @@ static void solve_mshift(qphix_gpu_eo_op_s *op, qphix_gpu_field_s **x, qphix_gpu
   memset(&ma, 0, sizeof(ma));
   ma.vh = (int)lat->vh;
   ma.nshift = ns;
-  ma.r = static_cast<qphix_gpu_field_s *>(r)->sarg();
   ma.p0 = static_cast<qphix_gpu_field_s *>(p0)->sarg();
+  for (int j = 0; j < batch; j++) ma.r[j] = static_cast<qphix_gpu_field_s *>(*rs[j])->sarg();
   for (int s = 0; s < ns; s++) {
     ma.x[s] = x[s]->sarg();
     ma.p[s] = static_cast<qphix_gpu_field_s *>(*ps[s])->sarg();
   }
   ma.state = ds;
+  ma.hist = hist;
   if (!S.done) {
+    const dim3 grid(nblocks_for(lat->vh));
+    // one batch: iteration j runs on r[j] and leaves its residual in
+    // r[(j + 1) % batch]; the update pass comes before the last iteration's
+    // Dslash overwrites r[0]
     auto step = [&] {
-      MShiftArgs m = ma;
-      m.x_only = 0;
-      launch_mshift(prec, m, dim3(nblocks_for(lat->vh)), lat->stream);
-      check_launch();
-      ApplyOpts o1;
-      o1.red_mask = RED_NORM_OUT;
-      o1.fin = FIN_MCG_D;
-      o1.state = ds;
-      eo_apply(op, mp, p0, isign, cb, o1);
-      ApplyOpts o2;
-      o2.post = POST_RAXPY;
-      o2.red_mask = RED_NORM_R;
-      o2.fin = FIN_MCG_R;
-      o2.state = ds;
-      o2.r = r;
-      eo_apply(op, mmp, mp, -isign, cb, o2);
+      for (int j = 0; j < batch; j++) {
+        launch_mshift_base(prec, (int)lat->vh, ns, j, ma.r[j], ma.p0, ds, hist, grid, lat->stream);
+        check_launch();
+        if (j == batch - 1) {
+          launch_mshift_update(prec, ma, grid, lat->stream);
+          check_launch();
+        }
+        ApplyOpts o1;
+        o1.red_mask = RED_NORM_OUT;
+        o1.fin = FIN_MCG_D;
+        o1.state = ds;
+        eo_apply(op, mp, p0, isign, cb, o1);
+        ApplyOpts o2;
+        o2.post = POST_RAXPY;
+        o2.red_mask = RED_NORM_R;
+        o2.fin = FIN_MCG_R;
+        o2.state = ds;
+        o2.r = *rs[j];
+        o2.x = *rs[(j + 1) % batch];
+        eo_apply(op, mmp, mp, -isign, cb, o2);
+      }
     };
-    std::string key = "mcg/" + std::to_string(op->serial) + "/" + fkey(r) + fkey(p0) + fkey(mp) + fkey(mmp) + "/";
+    std::string key = "mcg/" + std::to_string(op->serial) + "/" + fkey(p0) + fkey(mp) + fkey(mmp) + "/";
+    for (int j = 0; j < batch; j++) key += fkey(*rs[j]) + "r";
     for (int s = 0; s < ns; s++) key += fkey(x[s]) + "," + fkey(*ps[s]) + ";";
     key += "/" + std::to_string(isign) + std::to_string(cb);
-    run_iterations(lat, step, max_iters, key);
+    run_iterations(lat, step, max_iters, key, batch);
     mv += 2ul * lat->h_state->iter;
     // the x update of the last iteration is still pending
     MShiftArgs m = ma;
     m.x_only = 1;
-    launch_mshift(prec, m, dim3(nblocks_for(lat->vh)), lat->stream);
+    launch_mshift_update(prec, m, grid, lat->stream);
     check_launch();
     QPX_CUDA(cudaStreamSynchronize(lat->stream));
   }

@@ -76,7 +76,7 @@ __host__ __device__ inline bool is_two_flavour(int epi, int achi)
 enum Post : int {
   POST_STORE = 0,  // store out
   POST_CG = 1,     // r -= a out ; x += a p ; |r|^2   (a = state S_A[rhs]); out not stored
-  POST_RAXPY = 2,  // r += b out ; |r|^2             (b = state S_B[rhs]); out not stored
+  POST_RAXPY = 2,  // x = r + b out ; |x|^2          (b = state S_B[rhs]; x may be r); out not stored
 };
 // reduction value bits (values appear in this order)
 enum RedBit : int {
@@ -951,13 +951,13 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
       }
       if (a.post == POST_STORE) {
         L::store(a.out, rr, s, act, res[r]);
-      } else if (a.post == POST_RAXPY) {  // r += b mmp ; |r|^2
+      } else if (a.post == POST_RAXPY) {  // x = r + b mmp ; |x|^2
         const T cb_ = rhs_coef<RL, T>(st->v[S_B], rr);
         T rv[24];
         L::load(a.r, rr, s, rv);
 #pragma unroll
         for (int k = 0; k < 24; k++) rv[k] = mad(cb_, res[r][k], rv[k]);
-        L::store(a.r, rr, s, act, rv);
+        L::store(a.x, rr, s, act, rv);
         if constexpr (RL)
           red_norm_pair(rv, red[0][5], red[1][5]);
         else

@@ -68,6 +68,7 @@ struct qphix_gpu_lattice_s {
   double *h_result = nullptr;     // pinned mirror
   qpx::SolverState *state = nullptr;   // device
   qpx::SolverState *h_state = nullptr; // pinned mirror
+  void *mshift_hist = nullptr;          // device MShiftHist of multishift CG (lazy)
   void *grid_bar = nullptr;             // device GridBarrier of the persistent solvers (lazy)
   void *staging = nullptr;
   size_t staging_bytes = 0;
@@ -180,7 +181,9 @@ void launch_clover_in(int prec, Geom g, HostLayout L, const void *host, void *de
                       int nr, dim3 grid, cudaStream_t st);
 void launch_clover_out(int prec, Geom g, HostLayout L, void *host, const void *dev, long long stride, int vpc,
                        int nr, dim3 grid, cudaStream_t st);
-void launch_mshift(int prec, const MShiftArgs &a, dim3 grid, cudaStream_t st);
+void launch_mshift_base(int prec, int vh, int nshift, int slot, SpinorArg r, SpinorArg p0, const SolverState *state,
+                        MShiftHist *hist, dim3 grid, cudaStream_t st);
+void launch_mshift_update(int prec, const MShiftArgs &a, dim3 grid, cudaStream_t st);
 void launch_clover_build(int recon, int prec_out, Geom geo, GaugeArg g, void *out, long long stride, int vpc, int cb,
                          double diag_mass, double cr, double ct, dim3 grid, cudaStream_t st);
 void launch_clover_invert(int prec_in, int prec_out, Geom geo, const void *in, long long stride, int vpc_in, void *o0,
