@@ -1415,6 +1415,9 @@ extern "C" int qphix_gpu_clover_apply(qphix_gpu_field res, qphix_gpu_field chi, 
 // ===========================================================================
 // clover term construction / inversion on the device (clover_build.cu)
 // ===========================================================================
+// the clover kernels take 32 sites a block
+static dim3 clover_grid(const qphix_gpu_lattice_s *lat) { return dim3((unsigned)((lat->vh + 31) / 32)); }
+
 extern "C" int qphix_gpu_clover_build(qphix_gpu_field clov, qphix_gpu_field gauge, int cb, double diag_mass,
                                       double csw_r, double csw_t)
 {
@@ -1427,7 +1430,7 @@ extern "C" int qphix_gpu_clover_build(qphix_gpu_field clov, qphix_gpu_field gaug
     auto *lat = clov->lat;
     // tests/clover_term_qdp_w.h:133-137: the coefficients enter multiplied by 1/2
     launch_clover_build(gauge->recon, clov->prec, lat->geom(), gauge->garg(), clov->data, lat->stride, clov->spec.vpc,
-                        cb, diag_mass, 0.5 * csw_r, 0.5 * csw_t, dim3((unsigned)((lat->vh + 63) / 64)), lat->stream);
+                        cb, diag_mass, 0.5 * csw_r, 0.5 * csw_t, clover_grid(lat), lat->stream);
     check_launch();
   });
 }
@@ -1440,7 +1443,7 @@ extern "C" int qphix_gpu_clover_invert(qphix_gpu_field dst, qphix_gpu_field src)
     QPX_REQUIRE(same_shape(dst->lat, src->lat) && dst != src, "distinct fields of one lattice shape required");
     auto *lat = src->lat;
     launch_clover_invert(src->prec, dst->prec, lat->geom(), src->data, lat->stride, src->spec.vpc, dst->data, nullptr,
-                         dst->spec.vpc, 0, 0.0, dim3((unsigned)((lat->vh + 63) / 64)), lat->stream);
+                         dst->spec.vpc, 0, 0.0, clover_grid(lat), lat->stream);
     check_launch();
   });
 }
@@ -1488,7 +1491,7 @@ extern "C" int qphix_gpu_clover_invert_ndtm(qphix_gpu_field finv_up, qphix_gpu_f
     auto *lat = src->lat;
     launch_clover_invert(src->prec, finv_up->prec, lat->geom(), src->data, lat->stride, src->spec.vpc,
                          finv_up->data, finv_dn->data, finv_up->spec.vpc, 2, mu,
-                         dim3((unsigned)((lat->vh + 63) / 64)), lat->stream, clov_odiag->data, clov_odiag->spec.vpc,
+                         clover_grid(lat), lat->stream, clov_odiag->data, clov_odiag->spec.vpc,
                          eps);
     check_launch();
   });
@@ -1508,7 +1511,7 @@ extern "C" int qphix_gpu_clover_invert_twisted(qphix_gpu_field dst_plus, qphix_g
     auto *lat = src->lat;
     launch_clover_invert(src->prec, dst_plus->prec, lat->geom(), src->data, lat->stride, src->spec.vpc,
                          dst_plus->data, dst_minus->data, dst_plus->spec.vpc, 1, mu,
-                         dim3((unsigned)((lat->vh + 63) / 64)), lat->stream);
+                         clover_grid(lat), lat->stream);
     check_launch();
   });
 }
