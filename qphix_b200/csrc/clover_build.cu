@@ -105,15 +105,17 @@ __device__ __forceinline__ void dev_store_pair(void *base, long long stride, int
 //   Q - Q^+ = G - G^+,  G = U_mu(x) (S1 - S4) + (S2 - S3) U_mu(x-mu)
 // with the two-link completions S of the four leaves: 10 products of 3 x 3
 // matrices a plane instead of 12.
-// What bounds it: FP64 arithmetic (1080 fused products a plane and site, 120
-// us at 24^3x48 at the pipe's rate) and the occupancy its ~170 registers
-// leave.  One thread per site over all planes kept six F's, spilled to a
-// 928-byte stack and took 666 us there, 18-real links; build of both
-// checkerboards and one inverse (below) 2281 -> 1376 us.
+// What bounds it: the latency of the link loads and product chains at the
+// occupancy the registers leave (24^3x48, 18-real links: FP64 pipe 22 % busy
+// and 591 us at 182 registers and one block of 6 warps per multiprocessor;
+// two blocks of at most 168 registers, with 52 bytes spilled, 375 us; the
+// pipe's own time is 120 us).  One thread per site over all planes kept six
+// F's, spilled to a 928-byte stack and took 666 us there; both checkerboards'
+// terms and one inverse (below) went from 2254 to 929 us.
 constexpr int kPlanes = 6, kLeafSites = 32;
 
 template <int RECON, typename Q>
-__global__ void __launch_bounds__(kPlanes *kLeafSites)
+__global__ void __launch_bounds__(kPlanes *kLeafSites, 2)
     clover_build_kernel(Geom geo, GaugeArg g, void *out, long long stride, int vpc, int cb, double diag_mass,
                         double coeff_r, double coeff_t)
 {
