@@ -623,12 +623,27 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
   return launch_dslash(prec, recon, epi, achi, sh, nullptr, dim3(1), nullptr);
 }
 
-DslashShape default_shape(int prec, bool gen)
+// The shape of a configuration that has not been timed.  FP32 arithmetic
+// on 12-real links with an even number of right-hand sides: two of them per
+// thread, so that each link is loaded and rebuilt once for both -- in the
+// float2 lanes for 16-bit storage, as two scalars for FP32 storage, whose
+// lane form spills in the a chi - b D psi epilogues.  Otherwise one site and
+// one right-hand side; two sites per thread is behind both.  Measured, A^-1 D
+// psi / a chi - b D psi with its reductions, us: FP16 16^3x32 x 8 rhs lanes
+// 41 / 60, one site 44 / 62, two sites 52 / 64; FP32 the same, two rhs 51 /
+// 77, lanes 50 / 103, one site 53 / 91, two sites 69 / 97; one rhs, FP32
+// 16^3x32 one site 11 / 16, two sites 14 / 22; FP16 32^3x64 95 / 122, 110 / 135.
+DslashShape default_shape(int prec, bool gen, int recon, int nrhs)
 {
   DslashShape sh;
   sh.gen = gen;
-  // FP32 arithmetic: two sites per thread in float2 lanes (paired FP32 ops)
-  if (!gen && prec != PREC_F64) sh.SP = 2;
+  if (gen || prec == PREC_F64 || recon != 12 || nrhs % 2) return sh;
+  if (prec == PREC_F32) {
+    sh.R = 2;
+  } else {
+    sh.SP = 2;
+    sh.rl = true;
+  }
   return sh;
 }
 
@@ -657,7 +672,7 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     sh.R = 2;
     return sh;
   }
-  if (gen) return default_shape(prec, true);
+  if (gen) return default_shape(prec, true, recon, a.nrhs);
   // forced shapes (experiments and tests): QPHIX_GPU_RHS_LANES=1 selects two
   // right-hand sides in the float2 lanes of one site
   const char *fr = getenv("QPHIX_GPU_RHS_TILE"), *fs = getenv("QPHIX_GPU_SITES_PER_THREAD");
@@ -668,10 +683,9 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     sh.rl = true;
     if (shape_built(prec, recon, epi, achi, sh, a.nrhs)) return sh;
   } else if (fr || fs) {
-    DslashShape sh = default_shape(prec, false);
+    DslashShape sh;
     if (fr) sh.R = atoi(fr);
     if (fs) sh.SP = atoi(fs);
-    if (sh.R == 2 && !fs) sh.SP = 1;
     if (sh.R >= 1 && sh.SP >= 1 && shape_built(prec, recon, epi, achi, sh, a.nrhs)) return sh;
   }
   std::vector<DslashShape> cands;
@@ -688,7 +702,7 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     sh.rl = true;
     if (shape_built(prec, recon, epi, achi, sh, a.nrhs)) cands.push_back(sh);
   }
-  if (cands.size() <= 1) return cands.empty() ? default_shape(prec, false) : cands[0];
+  if (cands.size() <= 1) return cands.empty() ? default_shape(prec, false, recon, a.nrhs) : cands[0];
   const int red = tuned_reductions(a);
   const std::string key = tune_key(lat, prec, recon, epi, achi, a.nrhs, red);
   {
@@ -698,7 +712,14 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
   }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   QPX_CUDA(cudaStreamIsCapturing(lat->stream, &cap));
-  if (!tune_enabled() || cap != cudaStreamCaptureStatusNone) return default_shape(prec, false);
+  if (!tune_enabled() || cap != cudaStreamCaptureStatusNone) {
+    // a captured solver iteration whose reductions were never timed: the
+    // shape timed without them (the solve's first application), else the rule
+    std::lock_guard<std::mutex> g(g_tune_mu);
+    auto it = g_tune.find(tune_key(lat, prec, recon, epi, achi, a.nrhs, 0));
+    if (it != g_tune.end()) return it->second.sh;
+    return default_shape(prec, false, recon, a.nrhs);
+  }
 
   // time every candidate writing a scratch field, with the configuration's
   // reductions (into the lattice's workspace) but no finalize, no fused
