@@ -672,7 +672,11 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     sh.R = 2;
     return sh;
   }
-  if (gen) return default_shape(prec, true, recon, a.nrhs);
+  if (gen) {
+    DslashShape sh = default_shape(prec, true, recon, a.nrhs);
+    sh.phases = a.dir_mask == 0xFFu && !a.halo;
+    return sh;
+  }
   // forced shapes (experiments and tests): QPHIX_GPU_RHS_LANES=1 selects two
   // right-hand sides in the float2 lanes of one site
   const char *fr = getenv("QPHIX_GPU_RHS_TILE"), *fs = getenv("QPHIX_GPU_SITES_PER_THREAD");

@@ -14,7 +14,7 @@ inline void check_pdl(cudaError_t e)
   if (e != cudaSuccess) throw Error(QPHIX_GPU_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
 }
 
-template <typename P, int RECON, int R, int S, int SP, bool GEN, bool RL = false>
+template <typename P, int RECON, int R, int S, int SP, int GEN, bool RL = false>
 void launch_dslash_k(int epi, int achi, const DslashArgs &a, dim3 grid, cudaStream_t st)
 {
   dim3 block(QPX_BLOCK);
@@ -41,19 +41,19 @@ void launch_dslash_nd(int epi, int achi, const DslashArgs &a, dim3 grid, cudaStr
 {
   dim3 block(QPX_BLOCK);
   if (achi == ACHI_NONE && epi == EPI_NDTM)
-    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NDTM, ACHI_NONE, 2, S, 1, false>, grid, block, st, (long long)grid.x * grid.y, a));
+    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NDTM, ACHI_NONE, 2, S, 1, GEN_NONE>, grid, block, st, (long long)grid.x * grid.y, a));
   else if (epi == EPI_NONE && achi == ACHI_NDTM)
-    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_NDTM, 2, S, 1, false>, grid, block, st, (long long)grid.x * grid.y, a));
+    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_NDTM, 2, S, 1, GEN_NONE>, grid, block, st, (long long)grid.x * grid.y, a));
   else if (achi == ACHI_NONE && epi == EPI_NDFCLOV)
-    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NDFCLOV, ACHI_NONE, 2, S, 1, false>, grid, block, st, (long long)grid.x * grid.y, a));
+    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NDFCLOV, ACHI_NONE, 2, S, 1, GEN_NONE>, grid, block, st, (long long)grid.x * grid.y, a));
   else if (epi == EPI_NONE && achi == ACHI_NDCLOV)
-    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_NDCLOV, 2, S, 1, false>, grid, block, st, (long long)grid.x * grid.y, a));
+    check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_NDCLOV, 2, S, 1, GEN_NONE>, grid, block, st, (long long)grid.x * grid.y, a));
   else
     throw Error(QPHIX_GPU_EINVAL, "unsupported two-flavour dslash combination");
 }
 
 // isign is a template parameter: the projector signs become adds / subtracts
-template <typename P, int RECON, int R, int SP, bool GEN, bool RL = false>
+template <typename P, int RECON, int R, int SP, int GEN, bool RL = false>
 void launch_dslash_s(int epi, int achi, const DslashArgs *a, dim3 grid, cudaStream_t st)
 {
   if (!a) return;  // shape query
@@ -65,7 +65,7 @@ void launch_dslash_s(int epi, int achi, const DslashArgs *a, dim3 grid, cudaStre
 
 // The shapes built for storage P.  a == nullptr: only report whether the
 // shape exists.  Returns false for a shape that is not built.
-//   general path (dir mask, twisted phases): R = 1, SP = 1
+//   general path (dir mask, halo, twisted phases) and phases alone: R = 1, SP = 1
 //   fast path: R = 1 SP = 1 for every precision; for FP32 arithmetic also
 //   SP = 2 (both link kinds), R = 2 (12-real links) and two right-hand sides
 //   in the float2 lanes (rl, 12-real links, even nrhs)
@@ -89,36 +89,41 @@ bool launch_dslash_p(int recon, int epi, int achi, const DslashShape &sh, const 
     if constexpr (fp32) {
       if (sh.R != 1 || sh.SP != 2 || sh.gen || recon != 12) return false;
       if (a && a->nrhs % 2) return false;
-      launch_dslash_s<P, 12, 1, 2, false, true>(epi, achi, a, grid, st);
+      launch_dslash_s<P, 12, 1, 2, GEN_NONE, true>(epi, achi, a, grid, st);
       return true;
     }
     return false;
   }
   if (sh.gen) {
     if (sh.R != 1 || sh.SP != 1) return false;
+    if (sh.phases) {
+      recon == 12 ? launch_dslash_s<P, 12, 1, 1, GEN_PHASES>(epi, achi, a, grid, st)
+                  : launch_dslash_s<P, 18, 1, 1, GEN_PHASES>(epi, achi, a, grid, st);
+      return true;
+    }
     if (recon == 12)
-      launch_dslash_s<P, 12, 1, 1, true>(epi, achi, a, grid, st);
+      launch_dslash_s<P, 12, 1, 1, GEN_ALL>(epi, achi, a, grid, st);
     else
-      launch_dslash_s<P, 18, 1, 1, true>(epi, achi, a, grid, st);
+      launch_dslash_s<P, 18, 1, 1, GEN_ALL>(epi, achi, a, grid, st);
     return true;
   }
   if (sh.R == 1 && sh.SP == 1) {
     if (recon == 12)
-      launch_dslash_s<P, 12, 1, 1, false>(epi, achi, a, grid, st);
+      launch_dslash_s<P, 12, 1, 1, GEN_NONE>(epi, achi, a, grid, st);
     else
-      launch_dslash_s<P, 18, 1, 1, false>(epi, achi, a, grid, st);
+      launch_dslash_s<P, 18, 1, 1, GEN_NONE>(epi, achi, a, grid, st);
     return true;
   }
   if constexpr (fp32) {
     if (sh.R == 1 && sh.SP == 2) {
       if (recon == 12)
-        launch_dslash_s<P, 12, 1, 2, false>(epi, achi, a, grid, st);
+        launch_dslash_s<P, 12, 1, 2, GEN_NONE>(epi, achi, a, grid, st);
       else
-        launch_dslash_s<P, 18, 1, 2, false>(epi, achi, a, grid, st);
+        launch_dslash_s<P, 18, 1, 2, GEN_NONE>(epi, achi, a, grid, st);
       return true;
     }
     if (sh.R == 2 && sh.SP == 1 && recon == 12) {
-      launch_dslash_s<P, 12, 2, 1, false>(epi, achi, a, grid, st);
+      launch_dslash_s<P, 12, 2, 1, GEN_NONE>(epi, achi, a, grid, st);
       return true;
     }
   }

@@ -73,6 +73,7 @@ __host__ __device__ inline bool is_two_flavour(int epi, int achi)
 {
   return epi == EPI_NDTM || epi == EPI_NDFCLOV || achi == ACHI_NDTM || achi == ACHI_NDCLOV;
 }
+enum Gen : int { GEN_NONE = 0, GEN_ALL = 1, GEN_PHASES = 2 };
 enum Post : int {
   POST_STORE = 0,  // store out
   POST_CG = 1,     // r -= a out ; x += a p ; |r|^2   (a = state S_A[rhs]); out not stored
@@ -518,9 +519,11 @@ __device__ __forceinline__ void lanes_set(f2 &d, const double *v) { d = make_flo
 // R      right-hand sides per thread (SP = 1)
 // ISIGN  +1: D, -1: D^dagger
 // SP     lattice sites per thread: 1, or 2 in float2 lanes (FP32 arithmetic)
-// GEN    honour a.dir_mask and twisted boundary phases.  Without GEN every
-//        hop is taken and no phase applied: the hops are then straight-line
-//        code and the compiler can schedule every load early.
+// GEN    GEN_ALL honours a.dir_mask, halo faces and twisted boundary phases
+//        hop by hop, at run time.  GEN_NONE takes every hop without a phase:
+//        straight-line code, so the compiler can schedule every load early.
+//        GEN_PHASES takes every hop and multiplies each by its direction's
+//        phase (1 where it has none): straight-line as well.
 // RL     (with SP = 2, R = 1, fast path) the float2 lanes hold two
 //        right-hand sides of one site instead of two sites: links and
 //        clover terms are loaded once for both (RhsLanes).
@@ -536,11 +539,12 @@ __device__ __forceinline__ void lanes_set(f2 &d, const double *v) { d = make_flo
 // dslash_kernel runs it once per CUDA block; the persistent solver kernels
 // (qpx_persist.cuh) run it over all virtual blocks of a phase from a grid
 // that stays resident.
-template <typename P, int RECON, int EPI, int ACHI, int R, int ISIGN, int SP, bool GEN, bool RL = false>
+template <typename P, int RECON, int EPI, int ACHI, int R, int ISIGN, int SP, int GEN, bool RL = false>
 __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverState *st, int vblock, int nvblocks)
 {
   using L = typename std::conditional<RL, RhsLanes<P>, Lanes<P, SP>>::type;
   using T = typename L::T;
+  constexpr bool G = GEN == GEN_ALL, PH = GEN == GEN_PHASES;
   static_assert(SP == 1 || R == 1, "two sites per thread take one right-hand side");
   static_assert(!RL || (SP == 2 && R == 1 && !GEN), "right-hand-side lanes: SP = 2, R = 1, fast path");
   constexpr int RT = RL ? 2 : R;  // right-hand sides per thread
@@ -550,14 +554,11 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
   const int rhs0 = tile * RT;
   int s[SP];
   bool act[SP];
-  if (RL) {
+  if (RL || SP == 1) {
     s[0] = sblock * QPX_BLOCK + threadIdx.x;
     act[0] = s[0] < a.geom.vh;
     s[SP - 1] = s[0];
     act[SP - 1] = act[0];
-  } else if (SP == 1) {
-    s[0] = sblock * QPX_BLOCK + threadIdx.x;
-    act[0] = s[0] < a.geom.vh;
   } else {
     // each warp owns 64 consecutive sites: lane l takes sites l and l + 32,
     // so every load instruction of the warp reads 32 consecutive sites
@@ -589,7 +590,7 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
       int xh, y, z, t, par;
       const int sl = s[l];
       site_coords(g, sl, a.cb, xh, y, z, t, par);
-      if (GEN && l == 0 && a.halo) {
+      if (G && l == 0 && a.halo) {
         const int x = 2 * xh + par;
         hlast[0] = x + 1 == g.nx;
         hfirst[0] = x == 0;
@@ -634,9 +635,9 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
 
 #define QPX_HOP(MU)                                                                       \
   {                                                                                       \
-    const bool tw = GEN && ((a.tbc_mask >> MU) & 1);                                      \
+    const bool tw = PH || (G && ((a.tbc_mask >> MU) & 1));                                    \
     /* forward hop: U_mu(x) (1 - isign g) psi(x + mu) */                                  \
-    if (!GEN || (a.dir_mask & (1u << (2 * MU + 1)))) {                                    \
+    if (!G || (a.dir_mask & (1u << (2 * MU + 1)))) {                                    \
       cx<T> u[3][3];                                                                      \
       L::template load_link<RECON>(a.gauge, a.cb, MU, s, u);                              \
       T cf;                                                                               \
@@ -647,7 +648,7 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
         lanes_set(cf, c);                                                                 \
       }                                                                                   \
       /* halo: the next block's first slice along MU (general path, one site per thread) */ \
-      const bool ghf = GEN && ((a.halo >> MU) & 1) && hlast[MU];                          \
+      const bool ghf = G && ((a.halo >> MU) & 1) && hlast[MU];                          \
       int ixf[SP];                                                                        \
       _Pragma("unroll") for (int l = 0; l < SP; l++) ixf[l] = ghf ? hface[MU] : nb[MU][1][l]; \
       const cx<T> ph = {splat<T>(a.tbc[MU][0]), splat<T>(a.tbc[MU][1])};                  \
@@ -677,9 +678,9 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
       }                                                                                   \
     }                                                                                     \
     /* backward hop: U_mu(x - mu)^+ (1 + isign g) psi(x - mu) */                          \
-    if (!GEN || (a.dir_mask & (1u << (2 * MU)))) {                                        \
+    if (!G || (a.dir_mask & (1u << (2 * MU)))) {                                        \
       /* halo: the previous block's last slice along MU and its U_MU (general path) */    \
-      const bool ghb = GEN && ((a.halo >> MU) & 1) && hfirst[MU];                         \
+      const bool ghb = G && ((a.halo >> MU) & 1) && hfirst[MU];                         \
       int ixb[SP];                                                                        \
       _Pragma("unroll") for (int l = 0; l < SP; l++) ixb[l] = ghb ? hface[MU] : nb[MU][0][l]; \
       cx<T> u[3][3];                                                                      \
@@ -690,7 +691,7 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
         double c[SP];                                                                     \
         _Pragma("unroll") for (int l = 0; l < SP; l++) c[l] =                             \
             (MU < 3) ? a.coeff_s                                                          \
-                     : (tfirst[l] ? ((GEN && a.halo) ? a.coeff_t_bwd_edge : a.coeff_t_edge) \
+                     : (tfirst[l] ? ((G && a.halo) ? a.coeff_t_bwd_edge : a.coeff_t_edge) \
                                   : a.coeff_t);                                           \
         lanes_set(cf, c);                                                                 \
       }                                                                                   \
@@ -986,7 +987,7 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
     reduce_epilogue<RT>(a.red, a.nrhs, rhs0, red_slots(a.red.mask), red, sblock, nvblocks / ntiles);
 }
 
-template <typename P, int RECON, int EPI, int ACHI, int R, int ISIGN, int SP, bool GEN, bool RL = false>
+template <typename P, int RECON, int EPI, int ACHI, int R, int ISIGN, int SP, int GEN, bool RL = false>
 __global__ void QPX_DSLASH_BOUNDS dslash_kernel(const __grid_constant__ DslashArgs a)
 {
   pdl_wait();

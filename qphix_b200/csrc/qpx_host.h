@@ -159,7 +159,8 @@ void lattice_trim(qphix_gpu_lattice_s *L);
 // boundary phases).  Grid: ceil(Vh / (QPX_BLOCK SP)) site blocks x nrhs / R.
 struct DslashShape {
   int R = 1, SP = 1;
-  bool gen = false;
+  bool gen = false;     // the general path
+  bool phases = false;  // of it, boundary phases only
   bool rl = false;  // with R = 1, SP = 2: two right-hand sides of one site in the float2 lanes
 };
 // a == nullptr: report only whether the shape is built for (prec, recon)

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(QPX_BLOCK) cg_persistent_kernel(const __grid_c
     for (int half = 0; half < 2 && ok; half++) {
       const DslashArgs &da = a.d[2 * half], &db = a.d[2 * half + 1];
       for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-        dslash_block<PC, RECON, EPI, ACHI_NONE, 1, ISIGN, 1, false>(da, &sst, vb, nvb);
+        dslash_block<PC, RECON, EPI, ACHI_NONE, 1, ISIGN, 1, GEN_NONE>(da, &sst, vb, nvb);
         __syncthreads();
       }
       if (!grid_barrier(a.bar, target, 2 * half)) {
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(QPX_BLOCK) cg_persistent_kernel(const __grid_c
         break;
       }
       for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-        dslash_block<PC, RECON, EPI_NONE, ACHI, 1, ISIGN, 1, false>(db, &sst, vb, nvb);
+        dslash_block<PC, RECON, EPI_NONE, ACHI, 1, ISIGN, 1, GEN_NONE>(db, &sst, vb, nvb);
         __syncthreads();
       }
       if (!grid_barrier(a.bar, target, 2 * half + 1)) {
