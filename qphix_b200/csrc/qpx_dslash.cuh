@@ -667,7 +667,7 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
           L::load_raw(ghf ? a.ghost_fwd[MU] : a.in, rhs0 + r, ixf, psi, nrm);                 \
           project<MU, -ISIGN>(psi, h);                                                    \
         }                                                                                 \
-        if (tw || SP == 2) { /* SP = 2: the folded form costs registers (spills) */       \
+        if (tw || (SP == 2 && !RL)) { /* two sites: the folded form costs registers (spills) */ \
           scale_h(h, cf * nrm, tw, ph);                                                   \
           link_mult<false>(u, h, ch);                                                     \
           recons_add<MU, -ISIGN>(ch, acc[r]);                                             \
@@ -711,7 +711,7 @@ __device__ __forceinline__ void dslash_block(const DslashArgs &a, const SolverSt
           L::load_raw(ghb ? a.ghost_bwd[MU] : a.in, rhs0 + r, ixb, psi, nrm);                 \
           project<MU, ISIGN>(psi, h);                                                     \
         }                                                                                 \
-        if (tw || SP == 2) { /* SP = 2: the folded form costs registers (spills) */       \
+        if (tw || (SP == 2 && !RL)) { /* two sites: the folded form costs registers (spills) */ \
           scale_h(h, cf * nrm, tw, ph);                                                   \
           link_mult<true>(u, h, ch);                                                      \
           recons_add<MU, ISIGN>(ch, acc[r]);                                              \
