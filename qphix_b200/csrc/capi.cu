@@ -582,8 +582,8 @@ struct Tmp {
 // A shape (right-hand sides per thread R, sites per thread SP) is chosen per
 // (precision, links, epilogue, lattice, nrhs) the first time that Dslash runs
 // outside stream capture: every built shape is timed on a scratch output
-// (one warm-up and three timed launches each, CUDA events on the lattice's
-// stream) and the fastest is kept for the life of the process.  Launches
+// (two rounds of one warm-up and three timed launches each, CUDA events on
+// the lattice's stream) and the fastest is kept for the life of the process.  Launches
 // that differ only in their fused solver updates or reductions share the
 // entry.  QPHIX_GPU_TUNE=0 (or qphix_gpu_tune_enable(0)) switches timing off
 // and uses the default shape; QPHIX_GPU_RHS_TILE / QPHIX_GPU_SITES_PER_THREAD
@@ -748,7 +748,10 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     PdlOff() { pdl_suspended() = true; }
     ~PdlOff() { pdl_suspended() = false; }
   } pdl_off;
-  for (const auto &sh : cands) {
+  // two rounds over the candidates, the better time of each: a single round
+  // of three ~10 us launches takes a passing disturbance for a slow shape
+  for (size_t i = 0; i < 2 * cands.size(); i++) {
+    const DslashShape &sh = cands[i % cands.size()];
     dim3 grid = dslash_grid(lat, sh, a.nrhs);
     // a reducing launch is timed with the fold of its partials
     auto once = [&] {
