@@ -67,14 +67,12 @@ void launch_blas(int prec, const BlasArgs &a, dim3 grid, cudaStream_t st)
 // block of QPX_FOLD_THREADS threads, launched right after the producing
 // kernel on its stream, instantiated per finalize step (FIN) so that each
 // carries only its own recurrence.  The nres = nrhs x nval values share the
-// 32 warps, a group of G = max(1, 32 / nres) warps per value (further rounds
-// when nres > 32): lane l of warp g of a group adds site blocks 32 g + l,
-// 32 g + l + 32 G, ... in that order (an even number of blocks in pairs: 64 g
-// + 2 l, and the next one in a second sum, so that 512 blocks are one round
-// of eight loads in flight), then a shuffle tree per warp and the group's
-// warps in order.  Warp 0 then runs the finalize, a lane per right-hand side.  A solver state that is already done makes it write
-// nothing, as the producing kernel did.
-template <int FIN>
+// 32 warps (fold_groups); each lane adds its partials in a fixed order
+// (fold_lane, or in pairs: PAIRS, where fold_pairs says so), then a shuffle
+// tree per warp and the group's warps in order.  Warp 0 then runs the
+// finalize, a lane per right-hand side.  A solver state that is already done
+// makes it write nothing, as the producing kernel did.
+template <int FIN, bool PAIRS>
 __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg ra, SolverState *st, int nrhs,
                                                                 int nparts)
 {
@@ -103,7 +101,7 @@ __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg 
       sst.coupled = st->coupled;
     }
   }
-  const int G = nres >= 32 ? 1 : 32 / nres;
+  const int G = fold_groups(nres);
   const int vpr = 32 / G;  // values per round
   for (int v0 = 0; v0 < nres; v0 += vpr) {
     const int slot = wid / G, g = wid % G;
@@ -111,7 +109,7 @@ __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg 
     double acc = 0.0;
     if (slot < vpr && v < nres) {
       const double *p = ra.partials + (long long)v * nparts;  // value-major: coalesced across the lanes
-      if (nparts % 2 == 0) {  // every value's row starts on 16 bytes: two partials a load
+      if constexpr (PAIRS) {  // nparts is even: every value's row starts on 16 bytes
         double acc1 = 0.0;
 #pragma unroll 8
         for (int b = 2 * (32 * g + lane); b < nparts; b += 64 * G) {
@@ -121,8 +119,7 @@ __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg 
         }
         acc += acc1;
       } else {
-#pragma unroll 8
-        for (int b = 32 * g + lane; b < nparts; b += 32 * G) acc += __ldcg(p + b);
+        acc = fold_lane(p, nparts, g, G, lane);
       }
     }
     acc = warp_sum(acc);
@@ -164,8 +161,12 @@ __global__ void __launch_bounds__(QPX_FOLD_THREADS) fold_kernel(const ReduceArg 
 
 void launch_fold(const ReduceArg &ra, SolverState *state, int nrhs, int nparts, cudaStream_t st)
 {
-#define QPX_FOLD_CASE(F) \
-  case F: check_pdl_launch(launch_pdl(fold_kernel<F>, dim3(1), dim3(QPX_FOLD_THREADS), st, (long long)nparts * nrhs, ra, state, nrhs, nparts)); break;
+  const bool pairs = fold_pairs(nrhs * ra.nval, nparts);
+#define QPX_FOLD_CASE(F)                                                                                             \
+  case F:                                                                                                            \
+    check_pdl_launch(launch_pdl(pairs ? fold_kernel<F, true> : fold_kernel<F, false>, dim3(1),                       \
+                                dim3(QPX_FOLD_THREADS), st, (long long)nparts * nrhs, ra, state, nrhs, nparts));     \
+    break;
   switch (ra.fin) {
     QPX_FOLD_CASE(FIN_NONE)
     QPX_FOLD_CASE(FIN_CG_A)

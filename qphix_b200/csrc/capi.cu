@@ -2168,6 +2168,8 @@ static bool run_cg_persistent(qphix_gpu_lattice_s *lat, const std::vector<Captur
   pa.nrhs = nrhs;
   pa.vh = (int)lat->vh;
   pa.nsb = nblocks_for(lat->vh);
+  // the kernel folds in fold_kernel's unpaired order only
+  if (fold_pairs(nrhs * pa.d[1].red.nval, pa.nsb) || fold_pairs(nrhs * pa.d[3].red.nval, pa.nsb)) return false;
   if (!lat->grid_bar) QPX_CUDA(cudaMalloc(&lat->grid_bar, sizeof(GridBarrier)));
   pa.bar = static_cast<GridBarrier *>(lat->grid_bar);
   const int grid = (int)std::min<long long>((long long)per_sm * nsm, (long long)pa.nsb * nrhs);

@@ -101,22 +101,19 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier *b, unsigned int &targe
 }
 
 // The nrhs x nval values of one reduction, from partials [value][nsb], into
-// res: the per-value arithmetic of fold_kernel (G = max(1, 32 / nres) groups,
-// group g's lane l adding site blocks 32 g + l, 32 g + l + 32 G, ..., a
-// shuffle tree per group, the groups added in order).
+// res: fold_kernel's additions in fold_kernel's order (fold_lane of each of a
+// value's groups, a shuffle tree per group, the groups added in order).  A
+// reduction that fold_kernel would add in pairs is not run here (the host
+// sends such solves, of many more sites, to the graph path).
 __device__ __forceinline__ void fold_in_block(const ReduceArg &ra, int nrhs, int nsb, double *res)
 {
   const int nres = nrhs * ra.nval;
-  const int G = nres >= 32 ? 1 : 32 / nres;
+  const int G = fold_groups(nres);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int v = wid; v < nres; v += QPX_BLOCK / 32) {
     const double *p = ra.partials + (long long)v * nsb;
     double t = 0.0;
-    for (int g = 0; g < G; g++) {
-      double acc = 0.0;
-      for (int b = 32 * g + lane; b < nsb; b += 32 * G) acc += __ldcg(p + b);
-      t += warp_sum(acc);
-    }
+    for (int g = 0; g < G; g++) t += warp_sum(fold_lane(p, nsb, g, G, lane));
     if (lane == 0) res[v] = t;
   }
   __syncthreads();

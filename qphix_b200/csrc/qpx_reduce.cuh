@@ -161,4 +161,29 @@ __device__ __forceinline__ void reduce_epilogue(const ReduceArg &ra, int nrhs, i
 
 constexpr int QPX_FOLD_THREADS = 1024;
 
+// The fold's nres values share its 32 warps, a group of fold_groups(nres)
+// warps per value (further rounds when nres > 32).  fold_lane is the share of
+// lane `lane` of a group's warp g: site blocks 32 g + lane, 32 g + lane + 32 G,
+// ... in that order.
+__host__ __device__ inline int fold_groups(int nres) { return nres >= 32 ? 1 : 32 / nres; }
+__device__ __forceinline__ double fold_lane(const double *p, int nparts, int g, int G, int lane)
+{
+  double acc = 0.0;
+#pragma unroll 8
+  for (int b = 32 * g + lane; b < nparts; b += 32 * G) acc += __ldcg(p + b);
+  return acc;
+}
+// Where a lane has four loads or more, fold_kernel takes an even number of
+// partials two to a load instead (64 g + 2 lane and the one after it, in two
+// sums).  Measured, InvRichardsonMultiPrec with pairs / without: FP16 16^3x32
+// x 12 rhs (16 loads a lane) 54.5 / 57.0 ms, x 8 rhs 36.1 / 36.7 ms, BF16
+// 16^4 x 12 rhs (8 loads) 16.3 / 16.8 ms; with fewer loads, and in FP64 CG,
+// within the noise.  The paired loop takes 54 registers to the other's 32,
+// so it has a kernel of its own: where every fold ran it, FP64 CG of 480
+// sites took 3.5 % longer.
+__host__ __device__ inline bool fold_pairs(int nres, int nparts)
+{
+  return nparts % 2 == 0 && nparts / (32 * fold_groups(nres)) >= 4;
+}
+
 }  // namespace qpx

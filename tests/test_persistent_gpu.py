@@ -87,6 +87,25 @@ def test_persistent_matches_graph_path(api, oracle, prec, nrhs, monkeypatch):
         assert rel_l2(xp[i], xg[i]) < (1e-12 if prec == "f64" else 1e-5)
 
 
+@pytest.mark.parametrize("dims", [(8, 8, 8, 8), (4, 4, 8, 10)])  # 16 and 5 blocks of 128 sites
+@pytest.mark.parametrize("prec,nrhs", [("f64", 1), ("f64", 3), ("f32", 1), ("f32", 3)])
+def test_persistent_same_bits_as_graph_path(api, oracle, dims, prec, nrhs, monkeypatch):
+    """Both paths add the same partials in the same order, so with the graph
+    path's launches in the persistent kernel's shape (one site and one
+    right-hand side per thread) the solutions are the same bits."""
+    monkeypatch.setenv("QPHIX_GPU_RHS_TILE", "1")
+    monkeypatch.setenv("QPHIX_GPU_SITES_PER_THREAD", "1")
+    s = make_setup(dims, seed=79, gauge_kind="weak", mass=0.1)
+    lat, M, O, keep = _ops(api, oracle, s, "clover", prec, 12)
+    b = np.stack([F.gaussian_spinor(dims, 80 + i) for i in range(nrhs)])
+    rsd = 1e-10 if prec == "f64" else 1e-5
+    xp, ip, np_launch = _solve(api, lat, M, b, prec, "1", monkeypatch, rsd=rsd)
+    xg, ig, ng_launch = _solve(api, lat, M, b, prec, "0", monkeypatch, rsd=rsd)
+    assert np_launch < ng_launch
+    assert [i["n_iters"] for i in ip] == [i["n_iters"] for i in ig]
+    assert np.array_equal(xp, xg)
+
+
 def test_persistent_max_iters_and_restart(api, oracle, monkeypatch):
     """max_iters stops the persistent loop as it stops the graph path (status
     1, the same iterate), and a second solve on the same lattice reuses the
