@@ -178,9 +178,9 @@ __device__ __forceinline__ double fold_lane(const double *p, int nparts, int g, 
 // sums).  Measured, InvRichardsonMultiPrec with pairs / without: FP16 16^3x32
 // x 12 rhs (16 loads a lane) 54.5 / 57.0 ms, x 8 rhs 36.1 / 36.7 ms, BF16
 // 16^4 x 12 rhs (8 loads) 16.3 / 16.8 ms; with fewer loads, and in FP64 CG,
-// within the noise.  The paired loop takes 54 registers to the other's 32,
-// so it has a kernel of its own: where every fold ran it, FP64 CG of 480
-// sites took 3.5 % longer.
+// within the noise.  The two loops are kernels of their own, 32 registers
+// each: one kernel with both took 54, and FP64 CG of 480 sites, whose folds
+// add four partials, 3.5 % longer.
 __host__ __device__ inline bool fold_pairs(int nres, int nparts)
 {
   return nparts % 2 == 0 && nparts / (32 * fold_groups(nres)) >= 4;
