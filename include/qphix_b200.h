@@ -140,6 +140,8 @@ int qphix_gpu_launch_count(unsigned long long *out);
  * links, epilogue, lattice, nrhs) is timed over its built shapes (right-hand
  * sides per thread, lattice sites per thread) the first time it runs
  * outside CUDA-graph capture; the fastest shape is kept for the process.
+ * A configuration that has not been timed (tuning off, or first met inside
+ * a captured solver iteration) takes a shape by a rule on its sizes and types.
  * Entries are listed in key order.  sites_per_thread = 0 (with rhs_tile = 2)
  * denotes the shape that keeps two right-hand sides of one site in the
  * float2 lanes of a thread. */
@@ -147,6 +149,9 @@ int qphix_gpu_tune_enable(int enable);
 int qphix_gpu_tune_entries(int *count);
 int qphix_gpu_tune_entry(int index, char *key, size_t key_len, int *rhs_tile, int *sites_per_thread,
                          double *launch_us);
+/* The shape of the lattice's last Dslash launch (captured = 0), or of the
+ * last one that a solver captured into its iteration graph (captured = 1). */
+int qphix_gpu_lattice_dslash_shape(qphix_gpu_lattice lat, int captured, int *rhs_tile, int *sites_per_thread);
 
 /* ---- lattice (replaces Geometry<FT,V,S,c12>, include/qphix/geometry.h:130) */
 int qphix_gpu_lattice_create(const int latt_size[4], qphix_gpu_lattice *out);

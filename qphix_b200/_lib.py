@@ -84,6 +84,7 @@ _SIGS = {
     "qphix_gpu_init": ([I_], I_),
     "qphix_gpu_launch_count": ([C.POINTER(C.c_ulonglong)], I_),
     "qphix_gpu_tune_enable": ([I_], I_),
+    "qphix_gpu_lattice_dslash_shape": ([P, I_, C.POINTER(C.c_int), C.POINTER(C.c_int)], I_),
     "qphix_gpu_tune_entries": ([C.POINTER(C.c_int)], I_),
     "qphix_gpu_tune_entry": ([I_, C.c_char_p, C.c_size_t, C.POINTER(C.c_int), C.POINTER(C.c_int),
                               C.POINTER(C.c_double)], I_),

@@ -97,6 +97,14 @@ class Lattice:
     def set_stream(self, stream_handle: int):
         check(L._lib.qphix_gpu_lattice_set_stream(self.h, C.c_void_p(stream_handle)))
 
+    def dslash_shape(self, captured=False):
+        """(rhs_per_thread, sites_per_thread) of this lattice's last Dslash launch,
+        or of the last one a solver captured into its iteration graph; coded as
+        in tune_entries"""
+        r, sp = C.c_int(0), C.c_int(0)
+        check(L._lib.qphix_gpu_lattice_dslash_shape(self.h, 1 if captured else 0, C.byref(r), C.byref(sp)))
+        return r.value, sp.value
+
     # allocators (Geometry::allocCB*)
     def spinor(self, prec="f64", nrhs=1):
         return Field(self, L.SPINOR, PREC[prec], 0, nrhs)
@@ -800,7 +808,8 @@ def launch_count():
 # Dslash launch-shape autotuner
 # ---------------------------------------------------------------------------
 def tune_enable(enable=True):
-    """Switch timing of new Dslash configurations on or off (off: default shape)."""
+    """Switch timing of new Dslash configurations on or off (off: configurations
+    not timed before take the shape that the rule on sizes and types gives)."""
     lib()
     check(L._lib.qphix_gpu_tune_enable(1 if enable else 0))
 

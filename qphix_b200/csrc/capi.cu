@@ -623,26 +623,42 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
   return launch_dslash(prec, recon, epi, achi, sh, nullptr, dim3(1), nullptr);
 }
 
-// The shape of a configuration that has not been timed.  FP32 arithmetic
-// on 12-real links with an even number of right-hand sides: two of them per
-// thread, so that each link is loaded and rebuilt once for both -- in the
-// float2 lanes for 16-bit storage, as two scalars for FP32 storage, whose
-// lane form spills in the a chi - b D psi epilogues.  Otherwise one site and
-// one right-hand side; two sites per thread is behind both.  Measured, A^-1 D
-// psi / a chi - b D psi with its reductions, us: FP16 16^3x32 x 8 rhs lanes
-// 41 / 60, one site 44 / 62, two sites 52 / 64; FP32 the same, two rhs 51 /
-// 77, lanes 50 / 103, one site 53 / 91, two sites 69 / 97; one rhs, FP32
-// 16^3x32 one site 11 / 16, two sites 14 / 22; FP16 32^3x64 95 / 122, 110 / 135.
-DslashShape default_shape(int prec, bool gen, int recon, int nrhs)
+// The shape of a configuration that has not been timed: a rule on sizes and
+// types alone, so that a captured solver iteration whose reductions were never
+// timed sums the same number of partials in every process.  One site and one
+// right-hand side per thread, unless the launch still has two blocks per
+// multiprocessor (296 on B200) at two per thread; then
+// - 12-real links and an even number of right-hand sides: two of them per
+//   thread, so that each link is loaded and rebuilt once for both -- in the
+//   float2 lanes for 16-bit storage, as two scalars for FP32 storage, whose
+//   lane form spills in the a chi - b D psi epilogues;
+// - else two sites in the float2 lanes for BF16, whose one-site kernels spend
+//   more on conversions than those of the other formats.
+// Measured, clover a chi - b D psi with its two reductions and their fold, us:
+//   16^3x32 x 8 rhs, 12-real links, one site / two sites / two rhs / lanes:
+//   FP32 86 / 93 / 72 / 81, FP16 57 / 61 / 58 / 54, BF16 66 / 59 / 65 / 57,
+//   Q16 64 / 65 / 63 / 60, Q16 with FP32 links 63 / 83 / 64 / 60
+//   the same with 18-real links, one site / two sites: FP32 97 / 102, FP16
+//   58 / 60, BF16 67 / 60, Q16 64 / 64; 24^3x48 x 1, BF16 49 / 47
+//   around the line, FP32 one site / two rhs and FP16 one site / lanes:
+//   256 blocks (8^3x16 x 16) 13.9 / 16.2, 12.2 / 14.6; 324 blocks (12^3x24 x
+//   4) 18.7 / 15.6, 14.7 / 16.2; 512 blocks (16^3x32 x 4) 47.2 / 45.2,
+//   29.8 / 31.2 (its A^-1 D psi 21.4 / 19.4)
+DslashShape default_shape(const qphix_gpu_lattice_s *lat, int prec, bool gen, int recon, int nrhs)
 {
   DslashShape sh;
   sh.gen = gen;
-  if (gen || prec == PREC_F64 || recon != 12 || nrhs % 2) return sh;
-  if (prec == PREC_F32) {
-    sh.R = 2;
-  } else {
+  const long long blocks = (lat->vh + QPX_BLOCK - 1) / QPX_BLOCK * nrhs / 2;
+  if (gen || prec == PREC_F64 || blocks < 296) return sh;
+  if (recon == 12 && nrhs % 2 == 0) {
+    if (prec == PREC_F32) {
+      sh.R = 2;
+    } else {
+      sh.SP = 2;
+      sh.rl = true;
+    }
+  } else if (prec == PREC_BF16) {
     sh.SP = 2;
-    sh.rl = true;
   }
   return sh;
 }
@@ -673,7 +689,7 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     return sh;
   }
   if (gen) {
-    DslashShape sh = default_shape(prec, true, recon, a.nrhs);
+    DslashShape sh = default_shape(lat, prec, true, recon, a.nrhs);
     sh.phases = a.dir_mask == 0xFFu && !a.halo;
     return sh;
   }
@@ -706,7 +722,7 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
     sh.rl = true;
     if (shape_built(prec, recon, epi, achi, sh, a.nrhs)) cands.push_back(sh);
   }
-  if (cands.size() <= 1) return cands.empty() ? default_shape(prec, false, recon, a.nrhs) : cands[0];
+  if (cands.size() <= 1) return cands.empty() ? default_shape(lat, prec, false, recon, a.nrhs) : cands[0];
   const int red = tuned_reductions(a);
   const std::string key = tune_key(lat, prec, recon, epi, achi, a.nrhs, red);
   {
@@ -716,14 +732,8 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
   }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   QPX_CUDA(cudaStreamIsCapturing(lat->stream, &cap));
-  if (!tune_enabled() || cap != cudaStreamCaptureStatusNone) {
-    // a captured solver iteration whose reductions were never timed: the
-    // shape timed without them (the solve's first application), else the rule
-    std::lock_guard<std::mutex> g(g_tune_mu);
-    auto it = g_tune.find(tune_key(lat, prec, recon, epi, achi, a.nrhs, 0));
-    if (it != g_tune.end()) return it->second.sh;
-    return default_shape(prec, false, recon, a.nrhs);
-  }
+  if (!tune_enabled() || cap != cudaStreamCaptureStatusNone)
+    return default_shape(lat, prec, false, recon, a.nrhs);
 
   // time every candidate writing a scratch field, with the configuration's
   // reductions (into the lattice's workspace) but no finalize, no fused
@@ -796,6 +806,13 @@ extern "C" int qphix_gpu_tune_entries(int *count)
   });
 }
 
+// the rhs-lanes shape reads as two right-hand sides on 0 sites per thread
+static void report_shape(const DslashShape &sh, int *rhs_tile, int *sites_per_thread)
+{
+  if (rhs_tile) *rhs_tile = sh.rl ? 2 : sh.R;
+  if (sites_per_thread) *sites_per_thread = sh.rl ? 0 : sh.SP;
+}
+
 extern "C" int qphix_gpu_tune_entry(int index, char *key, size_t key_len, int *rhs_tile, int *sites_per_thread,
                                     double *launch_us)
 {
@@ -805,10 +822,17 @@ extern "C" int qphix_gpu_tune_entry(int index, char *key, size_t key_len, int *r
     auto it = g_tune.begin();
     std::advance(it, index);
     if (key && key_len) snprintf(key, key_len, "%s", it->first.c_str());
-    // the rhs-lanes shape reads as two right-hand sides on 0 sites per thread
-    if (rhs_tile) *rhs_tile = it->second.sh.rl ? 2 : it->second.sh.R;
-    if (sites_per_thread) *sites_per_thread = it->second.sh.rl ? 0 : it->second.sh.SP;
+    report_shape(it->second.sh, rhs_tile, sites_per_thread);
     if (launch_us) *launch_us = it->second.us;
+  });
+}
+
+extern "C" int qphix_gpu_lattice_dslash_shape(qphix_gpu_lattice lat, int captured, int *rhs_tile,
+                                              int *sites_per_thread)
+{
+  return guard([&] {
+    QPX_REQUIRE(lat, "null lattice");
+    report_shape(lat->last_shape[captured ? 1 : 0], rhs_tile, sites_per_thread);
   });
 }
 
@@ -848,6 +872,7 @@ static void dslash_launch(qphix_gpu_lattice_s *lat, int prec, int recon, int epi
     a.red.result = lat->result;
     a.red.nval = red_nval(a.red.mask);
   }
+  lat->last_shape[lat->capturing] = sh;
   const dim3 grid = dslash_grid(lat, sh, a.nrhs);
   if (!launch_dslash(prec, recon, epi, achi, sh, &a, grid, lat->stream))
     throw Error(QPHIX_GPU_EINVAL, "no Dslash kernel built for this precision / link / shape combination");
@@ -1958,13 +1983,16 @@ void run_iterations(qphix_gpu_lattice_s *lat, Step &&step, int max_iter, const s
     cudaGraph_t graph = nullptr;
     unsigned long long before = g_launches.load();
     QPX_CUDA(cudaStreamBeginCapture(lat->stream, cudaStreamCaptureModeThreadLocal));
+    lat->capturing = true;
     try {
       step();
     } catch (...) {
+      lat->capturing = false;
       cudaStreamEndCapture(lat->stream, &graph);
       if (graph) cudaGraphDestroy(graph);
       throw;
     }
+    lat->capturing = false;
     QPX_CUDA(cudaStreamEndCapture(lat->stream, &graph));
     nodes = g_launches.load() - before;  // captured, not run: counted per replay below
     g_launches -= nodes;

@@ -46,6 +46,16 @@ ChunkSpec spinor_spec(int prec);
 ChunkSpec gauge_spec(int prec, int recon);
 ChunkSpec clover_spec(int prec, int nreal);
 
+// Launch shape of the Dslash kernel: R right-hand sides per thread, SP
+// lattice sites per thread, gen = the general path (direction mask, twisted
+// boundary phases).  Grid: ceil(Vh / (QPX_BLOCK SP)) site blocks x nrhs / R.
+struct DslashShape {
+  int R = 1, SP = 1;
+  bool gen = false;     // the general path
+  bool phases = false;  // of it, boundary phases only
+  bool rl = false;  // with R = 1, SP = 2: two right-hand sides of one site in the float2 lanes
+};
+
 }  // namespace qpx
 
 struct qphix_gpu_lattice_s {
@@ -78,6 +88,8 @@ struct qphix_gpu_lattice_s {
   std::map<std::string, cudaGraphExec_t> graphs;
   std::map<std::string, unsigned long long> graph_nodes;
   std::vector<std::string> graph_order;
+  bool capturing = false;          // a solver's iteration is being captured
+  qpx::DslashShape last_shape[2];  // of the last Dslash launched, and captured
   qpx::Geom geom() const
   {
     qpx::Geom g;
@@ -154,15 +166,6 @@ int lattice_create_pooled(const int latt[4], cudaMemPool_t pool, qphix_gpu_latti
 void lattice_trim(qphix_gpu_lattice_s *L);
 
 // ---- dispatch (implemented per precision) ----------------------------------
-// Launch shape of the Dslash kernel: R right-hand sides per thread, SP
-// lattice sites per thread, gen = the general path (direction mask, twisted
-// boundary phases).  Grid: ceil(Vh / (QPX_BLOCK SP)) site blocks x nrhs / R.
-struct DslashShape {
-  int R = 1, SP = 1;
-  bool gen = false;     // the general path
-  bool phases = false;  // of it, boundary phases only
-  bool rl = false;  // with R = 1, SP = 2: two right-hand sides of one site in the float2 lanes
-};
 // a == nullptr: report only whether the shape is built for (prec, recon)
 bool launch_dslash(int prec, int recon, int epi, int achi, const DslashShape &sh, const DslashArgs *a, dim3 grid,
                    cudaStream_t st);

@@ -8,8 +8,9 @@
 // same stream, adds the partials of every value in a fixed order -- a group
 // of warps per value, lane l of warp g taking site blocks in a fixed stride,
 // then shuffle trees and the group's warps in order -- and runs a finalize
-// step on thread 0.  The order of every addition is fixed by the launch
-// shape, so results are bitwise reproducible run to run.
+// step on warp 0.  The order of every addition is fixed by the launch
+// shape, so a launch of the same shape gives the same bits; shapes that the
+// autotuner timed may differ between processes (QPHIX_GPU_TUNE=0: never).
 //
 // The finalize step updates a SolverState in device memory (Krylov scalars
 // alpha, beta, omega, rho, residual norms, convergence flags) so that a

@@ -53,7 +53,8 @@ def test_boundary_phases(oracle, dims, prec, recon):
 @pytest.mark.parametrize("recon", [18, 12])
 @pytest.mark.parametrize("nrhs", [1, 2, 3, 4])
 def test_untimed_shapes(oracle, prec, recon, nrhs):
-    """the shape rule with the autotuner off, reductions included"""
+    """the autotuner off, reductions included: the rule's shape for a lattice
+    of few blocks (its others: test_shapes_gpu.py)"""
     from qphix_b200 import api
     dims = (6, 4, 2, 6)
     s = make_setup(dims, seed=47, mass=0.1)
@@ -69,6 +70,7 @@ def test_untimed_shapes(oracle, prec, recon, nrhs):
         red = D.dslashAChiMinusBDPsiNorms(gr, gp, gc, u, A, 0.25, 1, 1)
     finally:
         api.tune_enable(True)
+    assert lat.dslash_shape() == (1, 1)
     got = gr.download().reshape(nrhs, -1, 4, 3)
     for i in range(nrhs):
         want = oracle.clov_achimbdpsi(L, psi[i], chi[i], s["gauge"], s["clov"][1], 0.25, 0.0, 1, 1)
