@@ -705,7 +705,8 @@ static DslashShape choose_shape(qphix_gpu_lattice_s *lat, int prec, int recon, i
   } else if (fr || fs) {
     DslashShape sh;
     if (fr) sh.R = atoi(fr);
-    if (fs) sh.SP = atoi(fs);
+    // the right-hand sides alone: two sites per thread where that is built
+    sh.SP = fs ? atoi(fs) : (prec != PREC_F64 && sh.R != 2 ? 2 : 1);
     if (sh.R >= 1 && sh.SP >= 1 && shape_built(prec, recon, epi, achi, sh, a.nrhs)) return sh;
   }
   std::vector<DslashShape> cands;

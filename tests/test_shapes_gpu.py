@@ -74,3 +74,24 @@ def test_captured_iteration_keeps_the_rule(gauge, prec, recon):
         api.zero(x)
         api.InvBiCGStab(M, 3)(x, b, 1e-3)
         assert lat.dslash_shape(captured=True) == rule(prec, recon, nrhs), nrhs
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32", "f16"])
+def test_forced_shapes(prec, monkeypatch):
+    """the variables, one at a time and together"""
+    from qphix_b200 import api
+    lat = api.Lattice((4, 4, 4, 4))
+    u = lat.gauge(prec, 12)
+    x, y = lat.spinor(prec, 2), lat.spinor(prec, 2)
+    D = api.Dslash(lat, -1.0, 1.0, 1.0)
+    one = {"f64": (1, 1)}
+    for tile, sites, lanes, want in (("1", None, None, one.get(prec, (1, 2))), ("2", None, None, one.get(prec, (2, 1))),
+                                     (None, "1", None, (1, 1)), (None, "2", None, one.get(prec, (1, 2))),
+                                     ("1", "1", None, (1, 1)), ("1", "2", None, one.get(prec, (1, 2))),
+                                     ("2", "1", None, one.get(prec, (2, 1))), (None, None, "1", one.get(prec, (2, 0)))):
+        with monkeypatch.context() as m:
+            for name, v in (("RHS_TILE", tile), ("SITES_PER_THREAD", sites), ("RHS_LANES", lanes)):
+                if v:
+                    m.setenv("QPHIX_GPU_" + name, v)
+            D.dslash(y, x, u, 1, 0)
+        assert lat.dslash_shape() == want, (tile, sites, lanes)
