@@ -368,6 +368,9 @@ int qphix_gpu_solve_mr(qphix_gpu_eo_op op, qphix_gpu_field x, qphix_gpu_field rh
  * reported as -1, like the reference). */
 int qphix_gpu_solve_mr_smoother(qphix_gpu_eo_op op, qphix_gpu_field x, qphix_gpu_field rhs, int n_iters,
                                 double omega, int isign, int cb, qphix_gpu_solve_info *info);
+/* Multishift CG.  Temporaries: n_shift + 5 spinors and up to 7 more (3 for
+ * fewer than four shifts), at most half of the free device memory, kept by
+ * the lattice for its next solve. */
 int qphix_gpu_solve_mshift_cg(qphix_gpu_eo_op op, qphix_gpu_field *x, qphix_gpu_field rhs, int n_shift,
                               const double *shifts, const double *rsd_target, int max_iters, int isign,
                               int cb, int *n_iters, double *rsd_sq_final, unsigned long *mv_apps);

@@ -68,11 +68,24 @@ extern "C" int qphix_gpu_launch_count(unsigned long long *out)
 static void lattice_release(qphix_gpu_lattice_s *L);
 static void field_free(qphix_gpu_field_s *f);
 
-// device memory of a lattice's fields: stream-ordered from its pool, or cudaMalloc
+static void pool_release(qphix_gpu_lattice_s *L);
+
+// device memory of a lattice's fields: stream-ordered from its pool, or
+// cudaMalloc.  What does not fit takes the memory of the solvers' idle
+// temporaries.
 static cudaError_t dev_alloc(qphix_gpu_lattice_s *L, void **p, size_t bytes)
 {
-  if (L->mempool) return cudaMallocFromPoolAsync(p, bytes, L->mempool, L->stream);
-  return cudaMalloc(p, bytes);
+  auto once = [&] {
+    cudaError_t e = L->mempool ? cudaMallocFromPoolAsync(p, bytes, L->mempool, L->stream) : cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // not the next launch's error
+    return e;
+  };
+  cudaError_t e = once();
+  if (e == cudaErrorMemoryAllocation && !L->pool_free.empty()) {
+    pool_release(L);
+    e = once();
+  }
+  return e;
 }
 
 static void dev_free(qphix_gpu_lattice_s *L, bool pooled, void *p)
@@ -121,13 +134,31 @@ int qpx::lattice_create_pooled(const int latt[4], cudaMemPool_t pool, qphix_gpu_
   });
 }
 
-void qpx::lattice_trim(qphix_gpu_lattice_s *L)
+// wait for the lattice's stream and drop its cached iteration graphs, which
+// hold pointers to solver temporaries
+static void drop_graphs(qphix_gpu_lattice_s *L)
 {
   QPX_CUDA(cudaStreamSynchronize(L->stream));
   for (auto &kv : L->graphs) cudaGraphExecDestroy(kv.second);
   L->graphs.clear();
   L->graph_nodes.clear();
   L->graph_order.clear();
+}
+
+// free the solver temporaries that no solve is using
+static void pool_release(qphix_gpu_lattice_s *L)
+{
+  drop_graphs(L);
+  for (auto *f : L->pool_free) {
+    L->pool_all.erase(std::find(L->pool_all.begin(), L->pool_all.end(), f));
+    field_free(f);
+  }
+  L->pool_free.clear();
+}
+
+void qpx::lattice_trim(qphix_gpu_lattice_s *L)
+{
+  drop_graphs(L);
   for (auto *f : L->pool_all) field_free(f);
   L->pool_all.clear();
   L->pool_free.clear();
@@ -3037,6 +3068,32 @@ extern "C" int qphix_gpu_solve_richardson(qphix_gpu_eo_op op_outer, qphix_gpu_eo
 // the next of `batch` residual buffers, p0 = r + a p0 is a kernel of its own,
 // and every shifted x / p update of `batch` iterations is one multi-vector
 // kernel (qpx_blas.cuh).
+//
+// Iterations per batch.  The update pass moves (4 ns + batch) / batch spinors
+// per iteration, and the residuals of a batch take batch - 1 spinors more than
+// a batch of one.  Batches of 1 / 2 / 4 / 8, a whole solve: 24^3x48 FP64, 16
+// shifts 57.5 / 40.6 / 32.4 / 28.2 ms; 24^4 FP64, 4 shifts 13.0 / 11.2 / 10.2 /
+// 9.8 ms, 1 shift 10.5 / 9.8 / 9.5 / 9.3 ms; 24^3x48 FP16, 16 shifts 2.84 /
+// 2.23 / 2.04 / 1.85 ms.  Fewer than four shifts get batches of four: eight
+// would gain 2 to 4 % for more spinors than all their vectors.  The additional
+// buffers take at most half of the memory that is free; those that earlier
+// solves left in the pool are there already.  QPHIX_GPU_MSHIFT_BATCH lowers
+// the batch (to a power of two).
+static int mshift_batch(const qphix_gpu_lattice_s *lat, const qphix_gpu_field_s *r, int ns)
+{
+  int batch = ns >= 4 ? QPX_MSHIFT_BATCH : QPX_MSHIFT_BATCH / 2;
+  if (const char *e = getenv("QPHIX_GPU_MSHIFT_BATCH"))
+    while (batch > 1 && batch > atoi(e)) batch /= 2;
+  int have = 0;
+  for (const auto *f : lat->pool_free) have += f->prec == r->prec && f->nrhs == 1;
+  if (batch - 1 > have) {
+    size_t free_bytes = 0, total = 0;
+    QPX_CUDA(cudaMemGetInfo(&free_bytes, &total));
+    while (batch - 1 > have && (size_t)(batch - 1 - have) * r->bytes > free_bytes / 2) batch /= 2;
+  }
+  return batch;
+}
+
 static void solve_mshift(qphix_gpu_eo_op_s *op, qphix_gpu_field_s **x, qphix_gpu_field_s *rhs, int ns,
                          const double *shifts, const double *rsd, int max_iters, int isign, int cb, int *n_iters,
                          double *rsd_sq_final, unsigned long *mv_apps)
@@ -3057,20 +3114,7 @@ static void solve_mshift(qphix_gpu_eo_op_s *op, qphix_gpu_field_s **x, qphix_gpu
   std::vector<std::unique_ptr<Tmp>> ps, rs;
   for (int s = 0; s < ns; s++) ps.emplace_back(new Tmp(lat, prec, 1));
   rs.emplace_back(new Tmp(lat, prec, 1));
-  // A residual buffer per iteration of a batch: the update pass moves
-  // (4 ns + batch) / batch spinors per iteration (24^3x48 FP64, 16 shifts:
-  // 586 us in batches of 1).  For few shifts the buffers would outnumber the
-  // vectors they save passes over.  A device that is full gets the batch
-  // that fits.
-  const int want = ns >= 4 ? QPX_MSHIFT_BATCH : QPX_MSHIFT_BATCH / 2;
-  try {
-    while ((int)rs.size() < want) rs.emplace_back(new Tmp(lat, prec, 1));
-  } catch (const Error &e) {
-    if (e.code != QPHIX_GPU_ENOMEM) throw;
-    cudaGetLastError();  // the failed allocation, not a launch's error
-  }
-  int batch = 1;
-  while (2 * batch <= (int)rs.size()) batch *= 2;
+  op_tmp(op, 1, lat);
   if (!lat->mshift_hist) QPX_CUDA(cudaMalloc(&lat->mshift_hist, sizeof(MShiftHist)));
   MShiftHist *hist = static_cast<MShiftHist *>(lat->mshift_hist);
   qphix_gpu_field_s *r = *rs[0];
@@ -3089,6 +3133,16 @@ static void solve_mshift(qphix_gpu_eo_op_s *op, qphix_gpu_field_s **x, qphix_gpu
   }
   eo_apply(op, mp, p0, isign, cb, ApplyOpts());
   eo_apply(op, mmp, mp, -isign, cb, ApplyOpts());
+  // everything that the solve cannot do without is allocated: now the optional buffers
+  int batch = mshift_batch(lat, r, ns);
+  try {
+    while ((int)rs.size() < batch) rs.emplace_back(new Tmp(lat, prec, 1));
+  } catch (const Error &e) {
+    if (e.code != QPHIX_GPU_ENOMEM) throw;
+    while (batch > (int)rs.size()) batch /= 2;
+    rs.resize(batch);
+    pool_release(lat);  // what a smaller batch does not use
+  }
   unsigned long mv = 2;
   double d = norm2_host(mp)[0];
   double b = -cp / d;
