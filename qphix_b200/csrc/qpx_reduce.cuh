@@ -105,7 +105,8 @@ __device__ __forceinline__ void store_partial(double *p, double v)
 }
 
 // TAIL: a thread per live value adds the warps' sums, side by side; without
-// it thread 0 adds them value by value.  The streaming kernels take it; in
+// it thread 0 adds them value by value.  The streaming kernels take it (0.5
+// to 0.7 % of an InvRichardsonMultiPrec solve of 8 or 12 right-hand sides); in
 // the Dslash kernels, at their register cap, it disturbs the launches that
 // reduce nothing (FP32 clover 24^3x48 +1 %).
 template <int R, bool TAIL = false>
@@ -177,11 +178,11 @@ __device__ __forceinline__ double fold_lane(const double *p, int nparts, int g, 
 // Where a lane has four loads or more, fold_kernel takes an even number of
 // partials two to a load instead (64 g + 2 lane and the one after it, in two
 // sums).  Measured, InvRichardsonMultiPrec with pairs / without: FP16 16^3x32
-// x 12 rhs (16 loads a lane) 54.5 / 57.0 ms, x 8 rhs 36.1 / 36.7 ms, BF16
-// 16^4 x 12 rhs (8 loads) 16.3 / 16.8 ms; with fewer loads, and in FP64 CG,
-// within the noise.  The two loops are kernels of their own, 32 registers
-// each: one kernel with both took 54, and FP64 CG of 480 sites, whose folds
-// add four partials, 3.5 % longer.
+// x 12 rhs (16 loads a lane) 54.2 / 57.2 ms, x 8 rhs 35.8 / 36.8 ms, BF16
+// 16^4 x 12 rhs (8 loads) 16.2 / 16.9 ms; with fewer loads, and in FP64 CG,
+// within the noise.  The two loops are kernels of their own, of 42 and 32
+// registers: one kernel with both took 54, and FP64 CG of 480 sites, whose
+// folds add four partials, 3.5 % longer.
 __host__ __device__ inline bool fold_pairs(int nres, int nparts)
 {
   return nparts % 2 == 0 && nparts / (32 * fold_groups(nres)) >= 4;
