@@ -717,7 +717,10 @@ class MInvCGMixed:
     """Multishift CG with low-precision iterations and a batched refinement of
     every shift to its target (qphix_gpu_solve_mshift_cg_mixed; no reference
     counterpart).  xs: one-rhs fields in M's precision; M_low: the same
-    operator on low-precision fields."""
+    operator on low-precision fields.  Every shift
+    meets its target by its true residual; in time it was behind MInvCG
+    wherever measured (B200, FP32 inside, 16^3x32 to 32^3x64: 1.1 to 1.3 times
+    as long with 4 shifts, 2.2 to 2.4 with 16)."""
 
     def __init__(self, M, M_low, max_iters, max_shifts=32):
         self.M, self.M_low, self.max_iters, self.max_shifts = M, M_low, max_iters, max_shifts

@@ -662,7 +662,7 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
 // - 12-real links and an even number of right-hand sides: two of them per
 //   thread, so that each link is loaded and rebuilt once for both -- in the
 //   float2 lanes for 16-bit storage, as two scalars for FP32 storage, whose
-//   lane form spills in the a chi - b D psi epilogues;
+//   lane form spills up to 212 bytes in the a chi - b D psi epilogues;
 // - else two sites in the float2 lanes for BF16, whose one-site kernels spend
 //   more on conversions than those of the other formats.
 // Measured, clover a chi - b D psi with its two reductions and their fold, us:

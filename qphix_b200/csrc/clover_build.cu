@@ -108,10 +108,10 @@ __device__ __forceinline__ void dev_store_pair(void *base, long long stride, int
 // What bounds it: the latency of the link loads and product chains at the
 // occupancy the registers leave (24^3x48, 18-real links: FP64 pipe 22 % busy
 // and 591 us at 182 registers and one block of 6 warps per multiprocessor;
-// two blocks of at most 168 registers, with 52 bytes spilled, 375 us; the
+// two blocks of at most 168 registers, with 52 bytes spilled, 364 us; the
 // pipe's own time is 120 us).  One thread per site over all planes kept six
 // F's, spilled to a 928-byte stack and took 666 us there; both checkerboards'
-// terms and one inverse (below) went from 2254 to 929 us.
+// terms and one inverse (below) went from 2254 to 927 us.
 constexpr int kPlanes = 6, kLeafSites = 32;
 
 template <int RECON, typename Q>
@@ -289,7 +289,7 @@ __device__ __forceinline__ zd packed_at(const void *in, long long stride, int vp
 // matrix is 24 registers a thread and every access is coalesced.  One thread
 // per site with the matrices and their inverses in local memory (3.6 KB of
 // stack) took 1025 us at 24^3x48 (FP64, mode 0), 18 times the term's and its
-// inverse's bytes.
+// inverse's bytes; this takes 222 us.
 constexpr int kInvertThreads = 12 * 32;
 
 // rows below the diagonal, and the diagonal, of column j of a packed block

@@ -291,12 +291,15 @@ __global__ void __launch_bounds__(QPX_BLOCK) blas_kernel(const BlasArgs a)
 // mshift_update_kernel applies the recorded updates of all shifts in one
 // pass, in order, with the residuals those iterations ran on (r[0 .. n-1],
 // each iteration's residual in a buffer of its own).
-// What bounds it: HBM.  One pass per iteration moves 4 n_shift + 1 spinors
-// (586 us at 24^3x48 FP64 with 16 shifts, 62 % of the solve, at the copy
-// rate); a pass per 8 iterations moves (4 n_shift + 8) / 8 of them per
-// iteration and does the same arithmetic on the same values: the solve went
-// from 53.4 to 27.8 ms (24^3x48, 16 shifts, FP64), the solutions unchanged
-// bit for bit (27.6 ms in batches of 16, for eight more buffers).
+// What bounds it: HBM.  With every shift active one pass per iteration moved
+// 4 n_shift + 3 spinors (586 us on average at 24^3x48 FP64 with 16 shifts,
+// 62 % of the solve); now the base update moves 3 an iteration and the pass
+// 4 n_shift + 8 per eight of them, with the same arithmetic on the same
+// values: the solve went from 53.4 to 27.8 ms (24^3x48, 16 shifts, FP64), the
+// solutions unchanged bit for bit (27.6 ms in batches of 16, for eight more
+// buffers).  16-bit storage rounds x and p once per batch instead of once per
+// iteration (24^3x48 FP16, 16 shifts: 2.84 ms in batches of one, 1.85 of
+// eight).
 constexpr int QPX_MAX_SHIFTS = 32;
 constexpr int QPX_MSHIFT_BATCH = 8;
 struct MShiftHist {

@@ -27,9 +27,12 @@
 // 16^3x32 x 8 rhs): one site per thread with 16-bit storage runs best at 4
 // blocks (at most 128 registers, which it fits without spilling; left free
 // it takes 135 and drops to 3 blocks, 13 % slower at 32^3x64); FP32 / FP64
-// storage, which sits at the HBM roofline with ~170-255 registers, keeps the
-// compiler free (1); two sites or two right-hand sides per thread with at
-// most 168 (3).
+// storage keeps the compiler free (1): FP64 takes up to 255 registers, FP32
+// 161-168 in the hops and 200-231 in most a chi - b D psi forms, two blocks
+// per SM.  That leaves large lattices near the HBM rate (24^3x48 and up);
+// one right-hand side at 16^3x32 in FP32, 512 blocks in 1.73 waves of two per
+// SM, is below it.  Two sites or two right-hand sides per thread: at most 168
+// (3).
 #ifndef QPX_MINB1
 #define QPX_MINB1 1
 #endif
@@ -523,7 +526,10 @@ __device__ __forceinline__ void lanes_set(f2 &d, const double *v) { d = make_flo
 //        hop by hop, at run time.  GEN_NONE takes every hop without a phase:
 //        straight-line code, so the compiler can schedule every load early.
 //        GEN_PHASES takes every hop and multiplies each by its direction's
-//        phase (1 where it has none): straight-line as well.
+//        phase (1 where it has none): straight-line as well.  Operators with
+//        phases, GEN_ALL / GEN_PHASES: FP32 clover 20x12x28x36 x 3 rhs 117 /
+//        100 us, FP64 Wilson 24^4 98 / 81 us; 1.10 (full clover, 16-bit
+//        spinors on FP32 links) to 1.35 times over all storage types.
 // RL     (with SP = 2, R = 1, fast path) the float2 lanes hold two
 //        right-hand sides of one site instead of two sites: links and
 //        clover terms are loaded once for both (RhsLanes).
