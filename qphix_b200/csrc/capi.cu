@@ -658,13 +658,13 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
 // types alone, so that a captured solver iteration whose reductions were never
 // timed sums the same number of partials in every process.  One site and one
 // right-hand side per thread, unless the launch still has two blocks per
-// multiprocessor (296 on B200) at two per thread; then
+// multiprocessor (296 on B200; the lanes of BF16, whose one-site kernels spend
+// more on conversions, one) at two per thread; then
 // - 12-real links and an even number of right-hand sides: two of them per
 //   thread, so that each link is loaded and rebuilt once for both -- in the
 //   float2 lanes for 16-bit storage, as two scalars for FP32 storage, whose
 //   lane form spills up to 212 bytes in the a chi - b D psi epilogues;
-// - else two sites in the float2 lanes for BF16, whose one-site kernels spend
-//   more on conversions than those of the other formats.
+// - else two sites in the float2 lanes for BF16.
 // Measured, clover a chi - b D psi with its two reductions and their fold, us:
 //   16^3x32 x 8 rhs, 12-real links, one site / two sites / two rhs / lanes:
 //   FP32 86 / 93 / 72 / 81, FP16 57 / 61 / 58 / 54, BF16 66 / 59 / 65 / 57,
@@ -674,14 +674,18 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
 //   around the line, FP32 one site / two rhs and FP16 one site / lanes:
 //   256 blocks (8^3x16 x 16) 13.9 / 16.2, 12.2 / 14.6; 324 blocks (12^3x24 x
 //   4) 18.7 / 15.6, 14.7 / 16.2; 512 blocks (16^3x32 x 4) 47.2 / 45.2,
-//   29.8 / 31.2 (its A^-1 D psi 21.4 / 19.4)
+//   29.8 / 31.2 (its A^-1 D psi 21.4 / 19.4); BF16 one site / lanes, us per
+//   operator application in InvRichardsonMultiPrec: 168 blocks (12x8x16x14 x
+//   4) 40.0 / 37.6, 192 (8^3x16 x 12) 44.1 / 41.7, 270 (12x12x10x8 x 12)
+//   42.0 / 39.9
 DslashShape default_shape(const qphix_gpu_lattice_s *lat, int prec, bool gen, int recon, int nrhs)
 {
   DslashShape sh;
   sh.gen = gen;
   const long long blocks = (lat->vh + QPX_BLOCK - 1) / QPX_BLOCK * nrhs / 2;
-  if (gen || prec == PREC_F64 || blocks < 296) return sh;
-  if (recon == 12 && nrhs % 2 == 0) {
+  const bool pairs = recon == 12 && nrhs % 2 == 0;
+  if (gen || prec == PREC_F64 || blocks < (pairs && prec == PREC_BF16 ? 148 : 296)) return sh;
+  if (pairs) {
     if (prec == PREC_F32) {
       sh.R = 2;
     } else {
