@@ -658,8 +658,8 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
 // types alone, so that a captured solver iteration whose reductions were never
 // timed sums the same number of partials in every process.  One site and one
 // right-hand side per thread, unless the launch still has two blocks per
-// multiprocessor (296 on B200; the lanes of BF16, whose one-site kernels spend
-// more on conversions, one) at two per thread; then
+// multiprocessor (296 on B200; BF16, whose one-site kernels spend more on
+// conversions, one) at two per thread; then
 // - 12-real links and an even number of right-hand sides: two of them per
 //   thread, so that each link is loaded and rebuilt once for both -- in the
 //   float2 lanes for 16-bit storage, as two scalars for FP32 storage, whose
@@ -673,18 +673,18 @@ bool shape_built(int prec, int recon, int epi, int achi, const DslashShape &sh, 
 //   58 / 60, BF16 67 / 60, Q16 64 / 64; 24^3x48 x 1, BF16 49 / 47
 //   around the line, FP32 one site / two rhs and FP16 one site / lanes:
 //   256 blocks (8^3x16 x 16) 13.9 / 16.2, 12.2 / 14.6; 324 blocks (12^3x24 x
-//   4) 18.7 / 15.6, 14.7 / 16.2; 512 blocks (16^3x32 x 4) 47.2 / 45.2,
+//   4) 18.7 / 15.6, 14.7 / 16.2; 1024 blocks (16^3x32 x 4) 47.2 / 45.2,
 //   29.8 / 31.2 (its A^-1 D psi 21.4 / 19.4); BF16 one site / lanes, us per
 //   operator application in InvRichardsonMultiPrec: 168 blocks (12x8x16x14 x
 //   4) 40.0 / 37.6, 192 (8^3x16 x 12) 44.1 / 41.7, 270 (12x12x10x8 x 12)
-//   42.0 / 39.9
+//   42.0 / 39.9; one site / two sites, 256 blocks (16^3x32 x 1) 38.0 / 36.1
 DslashShape default_shape(const qphix_gpu_lattice_s *lat, int prec, bool gen, int recon, int nrhs)
 {
   DslashShape sh;
   sh.gen = gen;
   const long long blocks = (lat->vh + QPX_BLOCK - 1) / QPX_BLOCK * nrhs / 2;
   const bool pairs = recon == 12 && nrhs % 2 == 0;
-  if (gen || prec == PREC_F64 || blocks < (pairs && prec == PREC_BF16 ? 148 : 296)) return sh;
+  if (gen || prec == PREC_F64 || blocks < (prec == PREC_BF16 ? 148 : 296)) return sh;
   if (pairs) {
     if (prec == PREC_F32) {
       sh.R = 2;

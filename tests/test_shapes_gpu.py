@@ -1,6 +1,6 @@
 """Which launch shape a Dslash takes: the rule for configurations that were not
 timed, on both sides of its line (296 blocks at two sites or right-hand sides
-per thread, 148 for BF16 pairs), with the autotuner off and inside a solver's captured iteration.
+per thread, 148 for BF16), with the autotuner off and inside a solver's captured iteration.
 Shapes read (right-hand sides, sites) per thread, lanes (2, 0)."""
 import numpy as np
 import pytest
@@ -15,7 +15,7 @@ DIMS = (16, 16, 16, 18)  # 288 blocks of 128 sites a right-hand side
 
 def rule(prec, recon, nrhs):
     pairs = recon == 12 and nrhs % 2 == 0
-    if prec == "f64" or 288 * nrhs // 2 < (148 if pairs and prec == "bf16" else 296):
+    if prec == "f64" or 288 * nrhs // 2 < (148 if prec == "bf16" else 296):
         return 1, 1
     if pairs:
         return (2, 1) if prec == "f32" else (2, 0)
