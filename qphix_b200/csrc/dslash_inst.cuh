@@ -14,22 +14,30 @@ inline void check_pdl(cudaError_t e)
   if (e != cudaSuccess) throw Error(QPHIX_GPU_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
 }
 
+// Four blocks of the 16-bit one-site kernels fit on a multiprocessor, two or
+// three of the others: half their number counts for programmatic dependent
+// launch, so that it starts where the launch fills the device once.  With it
+// from 296 blocks on, InvRichardsonMultiPrec with FP16 inside took 2 to 3 %
+// longer than the two-site form of fewer than 296 blocks (18x8x14x16 x 3 rhs,
+// us per operator application: 39.5, two sites 38.6, this 36.4; 16^3x20 x 1
+// 41.3, 41.2, 38.2).
 template <typename P, int RECON, int R, int S, int SP, int GEN, bool RL = false>
 void launch_dslash_k(int epi, int achi, const DslashArgs &a, dim3 grid, cudaStream_t st)
 {
-  dim3 block(QPX_BLOCK);
+  const long long size = (long long)grid.x * grid.y / (P::has_norm && SP == 1 && R == 1 ? 2 : 1);
+  auto go = [&](auto kernel) { check_pdl(launch_pdl(kernel, grid, dim3(QPX_BLOCK), st, size, a)); };
   if (achi == ACHI_NONE) {
     switch (epi) {
-    case EPI_NONE: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_NONE, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
-    case EPI_CLOV: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_CLOV, ACHI_NONE, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
-    case EPI_TMINV: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_TMINV, ACHI_NONE, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
-    case EPI_FCLOV: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_FCLOV, ACHI_NONE, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
+    case EPI_NONE: return go(dslash_kernel<P, RECON, EPI_NONE, ACHI_NONE, R, S, SP, GEN, RL>);
+    case EPI_CLOV: return go(dslash_kernel<P, RECON, EPI_CLOV, ACHI_NONE, R, S, SP, GEN, RL>);
+    case EPI_TMINV: return go(dslash_kernel<P, RECON, EPI_TMINV, ACHI_NONE, R, S, SP, GEN, RL>);
+    case EPI_FCLOV: return go(dslash_kernel<P, RECON, EPI_FCLOV, ACHI_NONE, R, S, SP, GEN, RL>);
     }
   } else if (epi == EPI_NONE) {
     switch (achi) {
-    case ACHI_ALPHA: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_ALPHA, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
-    case ACHI_CLOV: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_CLOV, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
-    case ACHI_TM: check_pdl(launch_pdl(dslash_kernel<P, RECON, EPI_NONE, ACHI_TM, R, S, SP, GEN, RL>, grid, block, st, (long long)grid.x * grid.y, a)); return;
+    case ACHI_ALPHA: return go(dslash_kernel<P, RECON, EPI_NONE, ACHI_ALPHA, R, S, SP, GEN, RL>);
+    case ACHI_CLOV: return go(dslash_kernel<P, RECON, EPI_NONE, ACHI_CLOV, R, S, SP, GEN, RL>);
+    case ACHI_TM: return go(dslash_kernel<P, RECON, EPI_NONE, ACHI_TM, R, S, SP, GEN, RL>);
     }
   }
   throw Error(QPHIX_GPU_EINVAL, "unsupported dslash epilogue combination");
